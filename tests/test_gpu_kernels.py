@@ -101,6 +101,27 @@ def test_linear(dtype, wdtype, shape):
     assert rel(logits, ref) < 1e-5
 
 
+# the last row count of the streaming form and the first of the tiles; rows and features one beside a tile's edge; an inner size
+# of one value, of a piece less one, and sizes that are cut among the CTAs of a cluster (few tiles, long rows), evenly or not
+@pytest.mark.parametrize("shape", [(8, 129, 1), (9, 33, 15), (1, 7, 4), (3, 31, 130), (16, 65, 1024), (17, 63, 1028), (128, 128, 2048),
+                                   (129, 127, 4100), (64, 64, 260), (333, 896, 1184), (2049, 520, 36)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_linear_plain_forms(dtype, shape):
+    """Sums of K products, each rounded to float32: the error of a sum is at most K 2^-24 of the sum of magnitudes, and the
+    rounding of a random sign pattern far less; 4 sqrt(K) 2^-24 of the root sum of squares bounds every value here."""
+    M, N, K = shape
+    b = native()
+    a, w = rnd(M, K, dtype=DT[dtype]), rnd(N, K)
+    ref = a.double() @ w.double().T
+    size = (a.double() ** 2) @ (w.double() ** 2).T                  # sum of squared products
+    out = torch.full((M, N), float("nan"), device=DEV)
+    b.linear(a, w, None, out, False)
+    assert float(((out.double() - ref).abs() / (size.sqrt() * 4 * (K ** 0.5 + 1) * 2 ** -24 + 1e-30)).max()) < 1
+    again = torch.empty_like(out)
+    b.linear(a, w, None, again, False)
+    assert torch.equal(out, again)
+
+
 @pytest.mark.parametrize("geom", [(5, 1, 48, 48), (6, 3, 32, 16), (8, 8, 128, 128), (2, 2, 256, 64)])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_rope_kv_write(dtype, geom):
