@@ -300,7 +300,7 @@ def linear_rope_kv(a, w, bias, qkv_buf, cos_sin, n_rot, positions, slots, q_out,
 ACT_CLAMPED_GLU = 5          # a gated pair only: see linear_glu
 ACTIVATIONS = {"silu": 0, "relu": 1, "gelu_tanh": 2, "relu2": 3, "none": 4}       # relu2: the square of relu
 ACT_GLU = 256               # added to an activation code: gated form of the grouped product
-MOE_TILE = 128              # places of one expert per tile of the grouped product ...
+MOE_TILE = 256              # places of one expert per tile of the grouped product ...
 MOE_TILE_FEW = 16           # ... and in steps of few tokens, whose blocks only stream weights: more, smaller tiles
 
 
@@ -308,6 +308,12 @@ def moe_tile(pairs: int) -> int:
     """Places per tile for a step with ``pairs`` (token, choice) pairs."""
     return MOE_TILE_FEW if pairs <= 512 else MOE_TILE
 
+
+
+def moe_wants_rows(pairs: int, dtype) -> bool:
+    """Whether the grouped product over gathered rows runs on tiles of many places in bfloat16, whose copies want the rows of
+    consecutive places one behind the other: it then asks for scratch to lay them out."""
+    return dtype == torch.bfloat16 and moe_tile(pairs) == MOE_TILE and hasattr(backend(), "lib")
 
 
 def _act(name: str) -> int:
@@ -576,18 +582,19 @@ def moe_group(ids, experts: int, order, tile_expert, tile_p0, tile_n, n_tiles) -
 
 
 def moe_gemm(a, w, out, act: str, order, src_div: int, scatter: bool, tile_expert, tile_p0, tile_n, n_tiles, pairs: int,
-             glu: bool = False, clamp=None) -> None:
+             glu: bool = False, clamp=None, rows=None) -> None:
     """Grouped product over the places of :func:`moe_group`: out[dst(p)] = act(a[src(p)] @ w[expert(p)].T) with
     w [E, N, K]; src(p) = order[p] // src_div if src_div else p; dst(p) = order[p] if scatter else p.  ``glu``: the rows
     of an expert's matrix alternate gate, up, and out [.., N / 2] = act(gate) * up; act "clamped" with ``clamp`` = (limit,
-    alpha, offset) as in :func:`linear_glu`."""
+    alpha, offset) as in :func:`linear_glu`.  ``rows`` (see :func:`moe_wants_rows`): scratch [pairs, K] of ``a``'s type."""
     _need(w.dim() == 3 and a.shape[1] == w.shape[2], "moe_gemm: shape mismatch")
+    _need(rows is None or (src_div and rows.dtype == a.dtype and rows.shape == (a.shape[0] * src_div, a.shape[1])), "moe_gemm: rows are [pairs, K] of the input's type")
     _need((act == "clamped") == (clamp is not None) and (clamp is None or glu), "moe_gemm: the clamped form is gated and comes with its constants")
     _need(out.shape[1] == (w.shape[1] // 2 if glu else w.shape[1]) and (not glu or w.shape[1] % 2 == 0), "moe_gemm: output width mismatch")
     code = (ACT_CLAMPED_GLU if act == "clamped" else _act(act)) | (ACT_GLU if glu else 0)
     backend().moe_gemm(a, w, out, code, order, int(src_div), bool(scatter), tile_expert, tile_p0,
                        tile_n, n_tiles, moe_max_tiles(int(pairs), w.shape[0]), moe_tile(int(pairs)),
-                       **({"clamp": tuple(float(x) for x in clamp)} if clamp is not None else {}))
+                       **({"clamp": tuple(float(x) for x in clamp)} if clamp is not None else {}), **({"rows": rows} if rows is not None else {}))
 
 
 def moe_combine(y, weights, out) -> None:

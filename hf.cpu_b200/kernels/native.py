@@ -724,12 +724,12 @@ class NativeBackend:
         self._check(self.lib.hfb_moe_sort(_p(ids), c_int(ids.numel()), c_int(experts), c_int(tile), _p(order), _p(tile_expert),
                                           _p(tile_p0), _p(tile_n), _p(n_tiles), self._stream()), "moe_sort")
 
-    def moe_gemm(self, a, w, out, act, order, src_div, scatter, tile_expert, tile_p0, tile_n, n_tiles, max_tiles, tile, clamp=None):
-        self._on_gpu(a, w, out, order, tile_expert, tile_p0, tile_n, n_tiles)
+    def moe_gemm(self, a, w, out, act, order, src_div, scatter, tile_expert, tile_p0, tile_n, n_tiles, max_tiles, tile, clamp=None, rows=None):
+        self._on_gpu(a, w, out, order, tile_expert, tile_p0, tile_n, n_tiles, rows)
         consts = tuple(c_float(x) for x in (clamp or (0.0, 0.0, 0.0)))
         self._check(self.lib.hfb_moe_gemm(_p(a), c_int(_dt(a)), _p(w), c_int(_dt(w)), _p(out), c_int(_dt(out)), c_int(act), *consts,
-                                          c_int(w.shape[1]), c_int(w.shape[2]), _p(order), c_int(src_div), c_int(1 if scatter else 0),
-                                          _p(tile_expert), _p(tile_p0), _p(tile_n), _p(n_tiles), c_int(max_tiles), c_int(tile),
+                                          c_int(a.shape[0]), c_int(w.shape[0]), c_int(w.shape[1]), c_int(w.shape[2]), _p(order), c_int(src_div), c_int(1 if scatter else 0),
+                                          _p(tile_expert), _p(tile_p0), _p(tile_n), _p(n_tiles), c_int(max_tiles), c_int(tile), _p(rows),
                                           self._stream()), "moe_gemm")
 
     def moe_combine(self, y, weights, out):

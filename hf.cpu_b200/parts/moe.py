@@ -152,9 +152,10 @@ class MoeFfn(FeedForward):
             kernels.moe_group(ids, self.n, order, *tiles, n_tiles)
         h = ctx.buf("moe_h", (P, self.F), xn.dtype)
         y = ctx.buf("moe_y", (P, self.E), xn.dtype if xn.dtype == torch.float32 else torch.float32)
+        rows = ctx.buf("moe_rows", (P, self.E), xn.dtype) if kernels.moe_wants_rows(P, xn.dtype) else None
         with kernels.phase("gate_up"):
             kernels.moe_gemm(xn, self.w_up, h, self.activation, order, self.top, False, *tiles, n_tiles, P, glu=self.gated,
-                             clamp=self.clamp)
+                             clamp=self.clamp, rows=rows)
         with kernels.phase("down"):
             kernels.moe_gemm(h, self.w_down, y, "none", order, 0, True, *tiles, n_tiles, P)
         if self.identity:

@@ -560,3 +560,69 @@ def test_decode_attention_merges_its_own_splits(geom):
             assert rel(out.float(), apart.float()) < 1e-2
             assert int(b._counters.abs().sum()) == 0
     kernels.check_device_errors()
+
+
+# places per expert at the edges of the tensor-core form's tiles (a chunk of 16 or 32 columns, a box of 32 rows, a tile of 256
+# places and one beside it), an expert without any; inner sizes of one piece, less and more; features beside a tile's edge
+@pytest.mark.parametrize("shape", [((1, 15, 16, 17, 0, 31, 32, 33, 400), 3, 128, 64), ((255, 256, 257, 513, 3), 2, 130, 200),
+                                   ((700, 0, 0, 12), 4, 24, 8), ((64, 511), 1, 520, 1032)])
+@pytest.mark.parametrize("act", ["none", "relu2", "silu", "clamped"])
+def test_grouped_product(shape, act):
+    """Both directions of a layer's experts: gathered rows into places of the lists, places into pairs.  Exact products of
+    bfloat16 values summed in float32: 4 sqrt(K) 2^-24 of the root sum of squares; times what an activation can add, and one
+    rounding to bfloat16 (2^-9) where the output is of that type."""
+    counts, top, N, Kd = shape
+    b = native()
+    E, P = len(counts), -(-sum(counts) // top) * top
+    T = P // top
+    ids = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)] + [torch.full((P - sum(counts),), E)])
+    ids = ids[torch.randperm(P, generator=torch.Generator().manual_seed(P))].to(torch.int32).to(DEV).view(T, top)
+    order = torch.empty(P, dtype=torch.int32, device=DEV)
+    tiles = [torch.empty(b.moe_max_tiles(P, E), dtype=torch.int32, device=DEV) for _ in range(3)]
+    n_tiles = torch.empty(1, dtype=torch.int32, device=DEV)
+    b.moe_group(ids, E, order, *tiles, n_tiles)
+    n = int(n_tiles)
+    assert sorted(order[:sum(counts)].tolist()) == [i for i, e in enumerate(ids.flatten().tolist()) if e < E]
+    got = [0] * E
+    for e, c in zip(tiles[0][:n].tolist(), tiles[2][:n].tolist()):
+        got[e] += c
+    assert got == list(counts)
+    a, w = rnd(T, Kd, dtype=torch.bfloat16), rnd(E, N, Kd, dtype=torch.bfloat16, scale=Kd ** -0.5)
+    glu = act in ("silu", "clamped")
+    clamp = (1.5, 1.7, 1.0) if act == "clamped" else None
+
+    def expected(z):
+        if act == "relu2":
+            return z.clamp_min(0) ** 2
+        if act == "silu":
+            return torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2]
+        if act == "clamped":
+            g, u = z[:, 0::2].clamp(max=1.5), z[:, 1::2].clamp(-1.5, 1.5)
+            return g * torch.sigmoid(1.7 * g) * (u + 1.0)
+        return z
+
+    bound = 4 * (Kd ** 0.5 + 1) * 2 ** -24
+    for src_div, scatter, rows, dt in ((top, False, a, torch.bfloat16), (0, True, rnd(P, Kd, dtype=torch.bfloat16, seed=5), torch.float32)):
+        space = {"rows": torch.empty(P, Kd, dtype=torch.bfloat16, device=DEV)} if src_div else {}
+        out = torch.full((P, N // 2 if glu else N), 7.0, dtype=dt, device=DEV)
+        b.moe_gemm(rows, w, out, act, order, src_div, scatter, *tiles, n_tiles, P, glu=glu, clamp=clamp, **space)
+        places = torch.arange(sum(counts), device=DEV)
+        pair = order[:sum(counts)].long()
+        x = rows[pair // top if src_div else places].double()
+        e = ids.flatten()[pair].long()
+        want = torch.empty(sum(counts), out.shape[1], dtype=torch.float64, device=DEV)
+        for i in range(E):
+            if counts[i]:
+                want[e == i] = expected(x[e == i] @ w[i].double().T)
+        at = pair if scatter else places
+        err = (out[at].double() - want).abs()
+        # (the factors of a gated pair and the square each carry the sums' error times the other factor, at most about 4 here)
+        slack = 16 * bound * float(x.square().sum(-1).mean().sqrt()) + (2 ** -8 if dt == torch.bfloat16 else 2 ** -22) * want.abs()
+        assert bool((err <= slack + 1e-12).all()), float((err - slack).max())
+        untouched = torch.ones(P, dtype=torch.bool, device=DEV)
+        untouched[at] = False
+        assert bool((out[untouched] == 7.0).all())                       # no row of a place that does not exist is written
+        again = torch.empty_like(out)
+        b.moe_gemm(rows, w, again, act, order, src_div, scatter, *tiles, n_tiles, P, glu=glu, clamp=clamp, **space)
+        assert torch.equal(out[at], again[at])
+    b.check_device_errors()
