@@ -78,6 +78,25 @@ __device__ __forceinline__ float4 plane_sum4(const float *p, int splits, size_t 
     return v;
 }
 
+// Four consecutive values (i a multiple of 4, the array aligned to four of its values).
+__device__ __forceinline__ float4 load_any4(const void *p, int dt, size_t i)
+{
+    if (dt == HFB_F32) return *(const float4 *)((const float *)p + i);
+    const uint2 u = *(const uint2 *)((const __nv_bfloat16 *)p + i);
+    const float2 lo = __bfloat1622float2(*(const __nv_bfloat162 *)&u.x), hi = __bfloat1622float2(*(const __nv_bfloat162 *)&u.y);
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ void store_any4(void *p, int dt, size_t i, float4 v)
+{
+    if (dt == HFB_F32) { *(float4 *)((float *)p + i) = v; return; }
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    uint2 u;
+    u.x = *(const unsigned *)&lo; u.y = *(const unsigned *)&hi;
+    *(uint2 *)((__nv_bfloat16 *)p + i) = u;
+}
+// Whether load_any4 / store_any4 may take the array (null: nothing will be read).
+inline bool aligned4(const void *p, int dt) { return ((uintptr_t)p & (dt == HFB_F32 ? 15 : 7)) == 0; }
+
 __device__ __forceinline__ float warp_sum(float v)
 {
 #pragma unroll

@@ -61,6 +61,59 @@ __global__ void dyt_residual_kernel(const TY *y, int splits, const void *bias, i
     }
 }
 
+// The same for steps of many tokens, which memory bounds: four columns a thread, one vector a thread and no loop over the
+// grid, so that all of a block's reads are in flight together (the scalar form above waits for one value after the other,
+// but spreads the few values of a step of single tokens over more threads).  The sums keep their order: the same bits.
+// Measured (B200): 2,048 tokens of 2,048 with the next norm and four experts' rows each 71 -> 24 us (5.2 TB/s), without the
+// experts 33 -> 13 us (from L2).
+__global__ void __launch_bounds__(256)
+dyt_residual_vec_kernel(const float *y, int splits, const void *bias, int bias_dt, const float *mix_y, const float *mix_w, int top,
+                        DytParams p, float *residual, int has_next, DytParams next, void *out, int out_dt, int M, int E)
+{
+    pdl_entry();
+    pdl_sync_small();
+    const size_t total = (size_t)M * E, i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (i >= total) return;
+    const size_t m = i / E;
+    const int c = (int)(i - m * E);
+    const float4 old = *(const float4 *)(residual + i);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (splits) v = plane_sum4(y + i, splits, total);
+    if (bias) {
+        const float4 b = load_any4(bias, bias_dt, c);
+        v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+    }
+    if (mix_y) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float *rows = mix_y + m * top * E + c, *w = mix_w + m * top;
+        for (int j0 = 0; j0 < top; j0 += 4) {
+            float4 r[4];
+            float f[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (j0 + j < top) { r[j] = *(const float4 *)(rows + (size_t)(j0 + j) * E); f[j] = w[j0 + j]; }
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (j0 + j < top) {
+                    acc.x = fmaf(f[j], r[j].x, acc.x); acc.y = fmaf(f[j], r[j].y, acc.y);
+                    acc.z = fmaf(f[j], r[j].z, acc.z); acc.w = fmaf(f[j], r[j].w, acc.w);
+                }
+        }
+        v.x += acc.x; v.y += acc.y; v.z += acc.z; v.w += acc.w;
+    }
+    const float alpha = load_any(p.alpha, p.dt, 0);
+    const float4 w = load_any4(p.w, p.dt, c), b = load_any4(p.b, p.dt, c);
+    const float4 r = make_float4(old.x + (tanhf(alpha * v.x) * w.x + b.x), old.y + (tanhf(alpha * v.y) * w.y + b.y),
+                                 old.z + (tanhf(alpha * v.z) * w.z + b.z), old.w + (tanhf(alpha * v.w) * w.w + b.w));
+    *(float4 *)(residual + i) = r;
+    if (has_next) {
+        const float alpha2 = load_any(next.alpha, next.dt, 0);
+        const float4 w2 = load_any4(next.w, next.dt, c), b2 = load_any4(next.b, next.dt, c);
+        store_any4(out, out_dt, i, make_float4(tanhf(alpha2 * r.x) * w2.x + b2.x, tanhf(alpha2 * r.y) * w2.y + b2.y,
+                                               tanhf(alpha2 * r.z) * w2.z + b2.z, tanhf(alpha2 * r.w) * w2.w + b2.w));
+    }
+}
+
 enum { ACT_SILU = 0, ACT_RELU = 1, ACT_GELU_TANH = 2, ACT_RELU2 = 3, ACT_NONE = 4 };
 
 __device__ __forceinline__ float activate(float z, int act)
@@ -161,7 +214,16 @@ extern "C" int hfb_dyt_residual(const void *y, int y_dt, int splits, const void 
         (has_next && (!alpha2 || !w2 || !b2 || !valid_dt(p2_dt) || !valid_dt(out_dt))))
         return fail(HFB_EINVAL, "dyt_residual: bad arguments");
     DytParams p{alpha, w, b, p_dt}, n{alpha2, w2, b2, p2_dt};
-    const unsigned blocks = blocks_for((size_t)M * E);
+    const size_t total = (size_t)M * E;
+    // four columns a thread from where that still gives every SM four blocks
+    if (total >= (size_t)148 * 4 * 1024 && (E & 3) == 0 && (splits == 0 || y_dt == HFB_F32) && aligned4(y, HFB_F32) && aligned4(bias, bias_dt) &&
+        aligned4(mix_y, HFB_F32) && aligned4(w, p_dt) && aligned4(b, p_dt) && aligned4(residual, HFB_F32) &&
+        (!has_next || (aligned4(w2, p2_dt) && aligned4(b2, p2_dt) && aligned4(out, out_dt)))) {
+        g_launch_err = launch_pdl(dyt_residual_vec_kernel, dim3((unsigned)((total / 4 + 255) / 256)), dim3(256), 0, (cudaStream_t)s, (const float *)y, splits, bias,
+                                  bias_dt, mix_y, mix_w, top, p, residual, has_next, n, out, out_dt, M, E);
+        return check_pdl_launch(g_launch_err, "dyt_residual");
+    }
+    const unsigned blocks = blocks_for(total);
     if (y_dt == HFB_F32) g_launch_err = launch_pdl(dyt_residual_kernel<float>, dim3(blocks), dim3(256), 0, (cudaStream_t)s, (const float *)y, splits, bias, bias_dt, mix_y, mix_w, top, p, residual, has_next, n, out, out_dt, M, E);
     else g_launch_err = launch_pdl(dyt_residual_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, (cudaStream_t)s, (const __nv_bfloat16 *)y, splits, bias, bias_dt, mix_y, mix_w, top, p, residual, has_next, n, out, out_dt, M, E);
     return check_pdl_launch(g_launch_err, "dyt_residual");

@@ -626,3 +626,37 @@ def test_grouped_product(shape, act):
         b.moe_gemm(rows, w, again, act, order, src_div, scatter, *tiles, n_tiles, P, glu=glu, clamp=clamp, **space)
         assert torch.equal(out[at], again[at])
     b.check_device_errors()
+
+
+# rows by columns on both sides of where steps of many tokens take four columns a thread (148 * 4,096 values), the
+# last block ragged, and a width that four does not divide
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("M,E,S,top,splits", [(296, 2044, 2, 4, 1), (297, 2044, 2, 4, 1), (300, 2046, 2, 2, 1), (1190, 512, 3, 5, 3), (150, 4100, 8, 1, 2),
+                                              (600, 1024, 1, 3, 0)])
+def test_stream_tails_of_many_tokens_are_those_of_few(dtype, M, E, S, top, splits):
+    """The Dynamic Tanh tail and the write-back of the streams' copies: every value is its own sums in one order, so a step
+    gives the bits that the same tokens give in small portions (whose values the tests against float64 cover)."""
+    b, dt = native(), DT[dtype]
+    y = rnd(max(splits, 1), M, E)
+    ey, wts, h = rnd(M * top, E, seed=1), torch.rand(M, top, device=DEV), rnd(M, E, dtype=dt, seed=2)
+    ids = torch.randint(0, 6, (M, top), device=DEV, dtype=torch.int32)
+    P = [(rnd(1, dtype=dt, seed=3 + i).abs() + 0.2, rnd(E, dtype=dt, seed=4 + i), rnd(E, dtype=dt, seed=5 + i)) for i in range(2)]
+    res, x = rnd(M, E, seed=7), rnd(M, S * E, seed=8)
+    scale, B, d_out, nxt = rnd(E, dtype=dt, seed=9), rnd(S, S, seed=10), rnd(S, seed=11), rnd(S, seed=12)
+
+    def run(lo, hi):
+        r, out = res[lo:hi].clone(), torch.empty(hi - lo, E, dtype=dt, device=DEV)
+        mix = (ey[lo * top:hi * top].contiguous(), wts[lo:hi].contiguous())
+        b.dyt_residual(y[0, lo:hi].contiguous() if splits else None, P[0], r, P[1], out, mix=mix)
+        plain = res[lo:hi].clone()
+        b.dyt_residual(y[0, lo:hi].contiguous(), P[0], plain)
+        xx, out2 = x[lo:hi].clone(), torch.empty(hi - lo, E, dtype=dt, device=DEV)
+        planes = y[:, lo:hi].contiguous()
+        sources = [(planes, splits, 0.7), (planes[:1].contiguous(), 1, 1.3)] if splits else []
+        b.hc_update(xx, S, sources, mix + (ids[lo:hi].contiguous(), 4, h[lo:hi].contiguous()), scale, B, d_out, nxt, P[1], out2)
+        return r, out, plain, xx, out2
+
+    whole = run(0, M)
+    parts = [run(lo, min(lo + 64, M)) for lo in range(0, M, 64)]
+    for i, got in enumerate(whole):
+        assert torch.equal(got, torch.cat([p[i] for p in parts])), i
