@@ -131,73 +131,139 @@ __global__ void conv_carry_kernel(const float *x, int splits, int x_stride, int 
     }
 }
 
-// The recurrence.  Block = (request, head, slice of value channels); L lanes share a column of S, each holding R of its
-// d entries in registers (entry i of the column sits in lane i / R).  q and k rows are [Hq heads of d] (head h reads head
-// h / (H / Hq)), a (the decays) [H heads of d], v and o [H heads of dv]; every row pointer comes with its own stride so
+// The recurrence.  Block = (request, head, slice of value channels); L lanes share C columns of S, each holding R of the
+// d entries of each in registers (entry i of a column sits in lane i / R).  q and k rows are [Hq heads of d] (head h reads
+// head h / (H / Hq)), a (the decays) [H heads of d], v and o [H heads of dv]; every row pointer comes with its own stride so
 // that the operands may be slices of wider product outputs.  beta_logit [T, beta_stride]: u = sigmoid(beta_logit) (v -
 // S^T k); NULL: u = v.
 //
-// The walk along the tokens is a chain of dependent steps, so what a step waits for decides the kernel's speed: the
-// operands of `ct` tokens at a time (the head's q, k and a rows, the block's slice of v, beta) come into shared memory by
-// cp.async, two chunks deep, and a step reads them from there instead of from global memory.  A row of d values lies in
-// shared memory as L groups of R with 4 floats between the groups, so that the lanes of a column read their 16-byte
-// pieces from different banks.  Only the state's update is a chain from token to token; a lane's piece of o = S^T q
-// goes to shared memory as it is, and the pieces of a chunk's tokens are summed (in lane order) and stored when the
-// chunk is done.
+// The walk along the tokens is a chain of dependent steps, so what a step waits for and how many instructions it takes
+// decide the kernel's speed: the operands of `ct` tokens at a time (the head's q, k and a rows, the block's slice of v,
+// beta) come into shared memory by cp.async (sixteen bytes a copy where the arrays allow: `wide`), two chunks deep, and a
+// step reads them from there; entries are worked on in pairs (fma.rn.f32x2: either half rounds as an fma of its own), and
+// beta's sigmoid is taken once a chunk.  A row of d values lies in shared memory as L groups of R with 4 floats between the
+// groups, so that the lanes of a column read their 16-byte pieces from different banks; entries behind d are zeros there.
+// Only the state's update is a chain from token to token; a lane's piece of o = S^T q goes to shared memory as it is, and
+// the pieces of a chunk's tokens are summed (in lane order) and stored when the chunk is done.
+// What bounds it: latencies of a step at seven warps an SM (115 instructions a warp and token, one in 4.9 cycles).  Two columns
+// a lane use every operand read twice.  Measured (B200, 16 heads of 128 x 128, requests of 777, 551, 324 and 97 tokens): without
+// / with the delta rule 499 / 618 us with one column a lane, scalar fma, selects for the entries behind d and copies of four
+// bytes; 229 / 319 us now; 256 threads 354 / 401 us with one column a lane, 321 / 397 us with two; 64 threads with four
+// columns 239 / 345 us.
 __device__ __forceinline__ void cp_async4(float *dst, const float *src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async16(float *dst, const float *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <int R, int L>
-__global__ void __launch_bounds__(256)
+typedef unsigned long long f32pair;
+__device__ __forceinline__ f32pair pair_of(float x, float y)
+{
+    f32pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 halves(f32pair v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32pair fma2(f32pair a, f32pair b, f32pair c)
+{
+    f32pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32pair mul2(f32pair a, f32pair b)
+{
+    f32pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+constexpr int SCAN_THREADS = 128;
+
+template <int R, int L, int C, bool DELTA>
+__global__ void __launch_bounds__(SCAN_THREADS)
 linear_scan_kernel(const float *q, int q_stride, const float *k, int k_stride, const float *v, int v_stride,
                    const float *a, int a_stride, const float *beta_logit, int beta_stride, float q_scale, float *state,
                    size_t slot_stride, const int32_t *cu_tokens, const int32_t *seq_slots, int n_slots, float *o,
-                   int o_stride, int H, int Hq, int d, int dv, int ct, int *err)
+                   int o_stride, int H, int Hq, int d, int dv, int ct, int wide, int wide_state, int *err)
 {
-    pdl_wait();                                      // (a long kernel: its successor is released when the walk is done)
     extern __shared__ float4 scan_smem4[];
     float *smem = (float *)scan_smem4;
-    constexpr int COLS = 256 / L, RS = L * (R + 4);              // columns of a block; floats of a padded row
+    constexpr int LC = SCAN_THREADS / L, COLS = LC * C, RS = L * (R + 4);      // columns of a block; floats of a padded row
     const int stage_floats = (ct * (3 * RS + COLS + 1) + 3) & ~3;
-    float *ob = smem + 2 * stage_floats;                         // [ct][256]: every lane's piece of o
+    float *ob = smem + 2 * stage_floats;                         // [ct][COLS * L]: every lane's pieces of o
+    for (int i = threadIdx.x; i < 2 * stage_floats; i += SCAN_THREADS) smem[i] = 0.f;        // (the entries behind d stay so)
+    pdl_wait();                                      // (a long kernel: its successor is released when the walk is done)
     const int seq = blockIdx.x, h = blockIdx.y;
-    const int lcol = threadIdx.x / L, col = blockIdx.z * COLS + lcol, part = threadIdx.x % L;
+    const int lcol = threadIdx.x / L, part = threadIdx.x % L, col0 = blockIdx.z * COLS;
     const int slot = seq_slots[seq];
     if (slot < 0 || slot >= n_slots) { if (threadIdx.x == 0) atomicOr(err, HFB_ERR_SLOT); return; }
     const int t0 = cu_tokens[seq], t1 = cu_tokens[seq + 1];
-    const bool live = col < dv;                                  // (lanes beyond the last column follow along on column 0)
-    const int cj = live ? col : 0;
     const int hq = h / (H / Hq);
     const int i0 = part * R;
-    float *sp = state + (size_t)slot * slot_stride + ((size_t)h * dv + cj) * d + i0;
-    float S[R];
+    float *sp[C];
+    bool live[C];
+    f32pair S[C][R / 2];
 #pragma unroll
-    for (int r = 0; r < R; r++) S[r] = (i0 + r < d) ? sp[r] : 0.f;
-    bool in[R];
+    for (int c = 0; c < C; c++) {
+        const int col = col0 + c * LC + lcol;
+        live[c] = col < dv;                                      // (lanes beyond the last column follow along on column 0)
+        sp[c] = state + (size_t)slot * slot_stride + ((size_t)h * dv + (live[c] ? col : 0)) * d + i0;
+        if (wide_state) {
 #pragma unroll
-    for (int r = 0; r < R; r++) in[r] = i0 + r < d;
+            for (int r = 0; r < R; r += 4) {
+                const float4 x = i0 + r < d ? *(const float4 *)(sp[c] + r) : make_float4(0.f, 0.f, 0.f, 0.f);
+                S[c][r / 2] = pair_of(x.x, x.y);
+                S[c][r / 2 + 1] = pair_of(x.z, x.w);
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r += 2) S[c][r / 2] = pair_of(i0 + r < d ? sp[c][r] : 0.f, i0 + r + 1 < d ? sp[c][r + 1] : 0.f);
+        }
+    }
+    __syncthreads();                                             // the zeros are in place
 
     auto issue = [&](int c) {
         float *st = smem + (c & 1) * stage_floats;
         const int tb = t0 + c * ct, n = min(ct, t1 - tb);
-        for (int idx = threadIdx.x; idx < n * d; idx += 256) {
-            const int tt = idx / d, i = idx - tt * d;
-            float *dst = st + tt * RS + (i / R) * (R + 4) + i % R;
-            cp_async4(dst, q + (size_t)(tb + tt) * q_stride + hq * d + i);
-            cp_async4(dst + ct * RS, k + (size_t)(tb + tt) * k_stride + hq * d + i);
-            cp_async4(dst + 2 * ct * RS, a + (size_t)(tb + tt) * a_stride + h * d + i);
-        }
         float *sv = st + 3 * ct * RS;
-        for (int idx = threadIdx.x; idx < n * COLS; idx += 256) {
-            const int tt = idx / COLS, c_ = idx % COLS, gc = blockIdx.z * COLS + c_;
-            cp_async4(sv + idx, v + (size_t)(tb + tt) * v_stride + h * dv + (gc < dv ? gc : 0));
+        if (wide) {
+            const int d4 = d >> 2;
+            for (int idx = threadIdx.x; idx < n * d4; idx += SCAN_THREADS) {
+                const int tt = idx / d4, i = (idx - tt * d4) * 4;
+                float *dst = st + tt * RS + (i / R) * (R + 4) + i % R;
+                cp_async16(dst, q + (size_t)(tb + tt) * q_stride + hq * d + i);
+                cp_async16(dst + ct * RS, k + (size_t)(tb + tt) * k_stride + hq * d + i);
+                cp_async16(dst + 2 * ct * RS, a + (size_t)(tb + tt) * a_stride + h * d + i);
+            }
+            for (int idx = threadIdx.x; idx < n * (COLS / 4); idx += SCAN_THREADS) {
+                const int tt = idx / (COLS / 4), c_ = idx % (COLS / 4) * 4, gc = col0 + c_;
+                cp_async16(sv + tt * COLS + c_, v + (size_t)(tb + tt) * v_stride + h * dv + (gc < dv ? gc : 0));
+            }
+        } else {
+            for (int idx = threadIdx.x; idx < n * d; idx += SCAN_THREADS) {
+                const int tt = idx / d, i = idx - tt * d;
+                float *dst = st + tt * RS + (i / R) * (R + 4) + i % R;
+                cp_async4(dst, q + (size_t)(tb + tt) * q_stride + hq * d + i);
+                cp_async4(dst + ct * RS, k + (size_t)(tb + tt) * k_stride + hq * d + i);
+                cp_async4(dst + 2 * ct * RS, a + (size_t)(tb + tt) * a_stride + h * d + i);
+            }
+            for (int idx = threadIdx.x; idx < n * COLS; idx += SCAN_THREADS) {
+                const int tt = idx / COLS, c_ = idx % COLS, gc = col0 + c_;
+                cp_async4(sv + idx, v + (size_t)(tb + tt) * v_stride + h * dv + (gc < dv ? gc : 0));
+            }
         }
-        if (beta_logit)
-            for (int idx = threadIdx.x; idx < n; idx += 256) cp_async4(sv + ct * COLS + idx, beta_logit + (size_t)(tb + idx) * beta_stride + h);
+        if (DELTA)
+            for (int idx = threadIdx.x; idx < n; idx += SCAN_THREADS) cp_async4(sv + ct * COLS + idx, beta_logit + (size_t)(tb + idx) * beta_stride + h);
         cp_async_commit();
     };
 
@@ -206,61 +272,93 @@ linear_scan_kernel(const float *q, int q_stride, const float *k, int k_stride, c
     for (int c = 0; c < n_chunks; c++) {
         if (c + 1 < n_chunks) { issue(c + 1); cp_async_wait<1>(); } else cp_async_wait<0>();
         __syncthreads();
-        const float *st = smem + (c & 1) * stage_floats;
+        float *st = smem + (c & 1) * stage_floats;
         const int tb = t0 + c * ct, n = min(ct, t1 - tb);
+        if (DELTA) {
+            float *sb = st + 3 * ct * RS + ct * COLS;
+            for (int idx = threadIdx.x; idx < n; idx += SCAN_THREADS) sb[idx] = sigmoid_f(sb[idx]);
+            __syncthreads();
+        }
 #pragma unroll 2
         for (int tt = 0; tt < n; tt++) {
-            float qa[R], ka[R], aa[R];
-            const float4 *rq = (const float4 *)(st + tt * RS + part * (R + 4));
-            const float4 *rk = (const float4 *)(st + (ct + tt) * RS + part * (R + 4));
-            const float4 *ra = (const float4 *)(st + (2 * ct + tt) * RS + part * (R + 4));
+            f32pair qa[R / 2], ka[R / 2], aa[R / 2];
+            const ulonglong2 *rq = (const ulonglong2 *)(st + tt * RS + part * (R + 4));
+            const ulonglong2 *rk = (const ulonglong2 *)(st + (ct + tt) * RS + part * (R + 4));
+            const ulonglong2 *ra = (const ulonglong2 *)(st + (2 * ct + tt) * RS + part * (R + 4));
 #pragma unroll
             for (int r4 = 0; r4 < R / 4; r4++) {
-                const float4 x = rq[r4], y = rk[r4], z = ra[r4];
-                qa[4 * r4] = x.x; qa[4 * r4 + 1] = x.y; qa[4 * r4 + 2] = x.z; qa[4 * r4 + 3] = x.w;
-                ka[4 * r4] = y.x; ka[4 * r4 + 1] = y.y; ka[4 * r4 + 2] = y.z; ka[4 * r4 + 3] = y.w;
-                aa[4 * r4] = z.x; aa[4 * r4 + 1] = z.y; aa[4 * r4 + 2] = z.z; aa[4 * r4 + 3] = z.w;
+                const ulonglong2 x = rq[r4], y = rk[r4], z = ra[r4];
+                qa[2 * r4] = x.x; qa[2 * r4 + 1] = x.y;
+                ka[2 * r4] = y.x; ka[2 * r4 + 1] = y.y;
+                aa[2 * r4] = z.x; aa[2 * r4 + 1] = z.y;
             }
+            float u[C];
 #pragma unroll
-            for (int r = 0; r < R; r++) {                         // beyond d the shared memory holds nothing
-                qa[r] = in[r] ? qa[r] : 0.f; ka[r] = in[r] ? ka[r] : 0.f; aa[r] = in[r] ? aa[r] : 0.f;
-            }
-            const float vt = st[3 * ct * RS + tt * COLS + lcol];
-            float u = vt;
-            if (beta_logit) {
-                const float gate = sigmoid_f(st[3 * ct * RS + ct * COLS + tt]);
-                float dot4[4] = {0.f, 0.f, 0.f, 0.f};                // four chains, summed in a fixed order
+            for (int c_ = 0; c_ < C; c_++) u[c_] = st[3 * ct * RS + tt * COLS + c_ * LC + lcol];
+            if (DELTA) {
+                const float gate = st[3 * ct * RS + ct * COLS + tt];
+                float dot[C];
 #pragma unroll
-                for (int r = 0; r < R; r++) { S[r] *= aa[r]; dot4[r & 3] = fmaf(S[r], ka[r], dot4[r & 3]); }
-                float dot = (dot4[0] + dot4[1]) + (dot4[2] + dot4[3]);
+                for (int c_ = 0; c_ < C; c_++) {
+                    f32pair d01 = 0, d23 = 0;                        // four chains, summed in a fixed order
 #pragma unroll
-                for (int m = L / 2; m > 0; m >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, m);
-                u = gate * (vt - dot);
+                    for (int r = 0; r < R / 2; r += 2) {
+                        S[c_][r] = mul2(S[c_][r], aa[r]);
+                        d01 = fma2(S[c_][r], ka[r], d01);
+                        S[c_][r + 1] = mul2(S[c_][r + 1], aa[r + 1]);
+                        d23 = fma2(S[c_][r + 1], ka[r + 1], d23);
+                    }
+                    const float2 x = halves(d01), y = halves(d23);
+                    dot[c_] = (x.x + x.y) + (y.x + y.y);
+                }
 #pragma unroll
-                for (int r = 0; r < R; r++) S[r] = fmaf(ka[r], u, S[r]);
+                for (int m = L / 2; m > 0; m >>= 1)
+#pragma unroll
+                    for (int c_ = 0; c_ < C; c_++) dot[c_] += __shfl_xor_sync(0xffffffffu, dot[c_], m);
+#pragma unroll
+                for (int c_ = 0; c_ < C; c_++) {
+                    u[c_] = gate * (u[c_] - dot[c_]);
+                    const f32pair uu = pair_of(u[c_], u[c_]);
+#pragma unroll
+                    for (int r = 0; r < R / 2; r++) S[c_][r] = fma2(ka[r], uu, S[c_][r]);
+                }
             } else {
 #pragma unroll
-                for (int r = 0; r < R; r++) S[r] = fmaf(aa[r], S[r], ka[r] * u);
-            }
-            float acc4[4] = {0.f, 0.f, 0.f, 0.f};
+                for (int c_ = 0; c_ < C; c_++) {
+                    const f32pair uu = pair_of(u[c_], u[c_]);
 #pragma unroll
-            for (int r = 0; r < R; r++) acc4[r & 3] = fmaf(S[r], qa[r], acc4[r & 3]);
-            ob[tt * 256 + threadIdx.x] = (acc4[0] + acc4[1]) + (acc4[2] + acc4[3]);
+                    for (int r = 0; r < R / 2; r++) S[c_][r] = fma2(aa[r], S[c_][r], mul2(ka[r], uu));
+                }
+            }
+#pragma unroll
+            for (int c_ = 0; c_ < C; c_++) {
+                f32pair s01 = 0, s23 = 0;
+#pragma unroll
+                for (int r = 0; r < R / 2; r += 2) { s01 = fma2(S[c_][r], qa[r], s01); s23 = fma2(S[c_][r + 1], qa[r + 1], s23); }
+                const float2 x = halves(s01), y = halves(s23);
+                ob[tt * (COLS * L) + c_ * SCAN_THREADS + threadIdx.x] = (x.x + x.y) + (y.x + y.y);
+            }
         }
         __syncthreads();                                         // the stage is free for the chunk after the next
-        for (int idx = threadIdx.x; idx < n * COLS; idx += 256) {
-            const int tt = idx / COLS, c_ = idx % COLS, gc = blockIdx.z * COLS + c_;
+        for (int idx = threadIdx.x; idx < n * COLS; idx += SCAN_THREADS) {
+            const int tt = idx / COLS, c_ = idx % COLS, gc = col0 + c_;
+            const float4 *piece = (const float4 *)(ob + tt * (COLS * L) + c_ * L);
             float acc = 0.f;
 #pragma unroll
-            for (int l = 0; l < L; l++) acc += ob[tt * 256 + c_ * L + l];
+            for (int l = 0; l < L / 4; l++) { const float4 x = piece[l]; acc += x.x; acc += x.y; acc += x.z; acc += x.w; }
             if (gc < dv) o[(size_t)(tb + tt) * o_stride + h * dv + gc] = acc * q_scale;
         }
     }
     pdl_trigger();
-    if (live) {
 #pragma unroll
-        for (int r = 0; r < R; r++)
-            if (i0 + r < d) sp[r] = S[r];
+    for (int c = 0; c < C; c++) {
+        if (!live[c]) continue;
+#pragma unroll
+        for (int r = 0; r < R; r += 2) {
+            const float2 x = halves(S[c][r / 2]);
+            if (i0 + r < d) sp[c][r] = x.x;
+            if (i0 + r + 1 < d) sp[c][r + 1] = x.y;
+        }
     }
 }
 
@@ -491,22 +589,36 @@ extern "C" int hfb_linear_scan(const float *q, int q_stride, const float *k, int
         return fail(HFB_EINVAL, "linear_scan: bad arguments (H=%d Hq=%d d=%d dv=%d)", H, Hq, d, dv);
     if (d > REC_MAX_D) return fail(HFB_ENOTSUP, "linear_scan: key heads above %d are not supported", REC_MAX_D);
     if (H > 65535) return fail(HFB_ENOTSUP, "linear_scan: %d heads exceed the grid limit", H);
-    // tokens per chunk: two stages of ct * (3 padded rows + the columns' values + beta) floats and the lanes' pieces of o
-    // (ct * 256 floats) within 46 KB, 16 at most
-#define HFB_SCAN(R, L) do { \
-        const int per_token = (3 * L * (R + 4) + 256 / L + 1) * 4; \
-        int ct = (46 * 1024 - 32) / (2 * per_token + 1024); \
-        ct = ct < 1 ? 1 : (ct > 16 ? 16 : ct); \
-        const size_t smem = 2 * (size_t)(((ct * (per_token / 4)) + 3) & ~3) * 4 + (size_t)ct * 1024; \
-        g_launch_err = launch_pdl(linear_scan_kernel<R, L>, dim3(S, H, (dv + 256 / L - 1) / (256 / L)), dim3(256), smem, (cudaStream_t)s, q, q_stride, \
+    // sixteen bytes a copy where every row of the operands (and of the state) starts and ends on such a piece
+    const bool wide = (d & 3) == 0 && (dv & 3) == 0 && ((q_stride | k_stride | v_stride | a_stride) & 3) == 0 && aligned4(q, HFB_F32) &&
+                      aligned4(k, HFB_F32) && aligned4(v, HFB_F32) && aligned4(a, HFB_F32);
+    const bool wide_state = (d & 3) == 0 && (slot_stride & 3) == 0 && aligned4(state, HFB_F32);
+    // tokens per chunk, 16 at most: two stages of ct * (3 padded rows + the columns' values + beta) floats and the lanes' pieces
+    // of o within 84 KB (two blocks an SM)
+#define HFB_SCAN_LAUNCH(R, L, C, DELTA) do { \
+        constexpr int COLS = SCAN_THREADS / L * C; \
+        const int per_token = (3 * L * (R + 4) + COLS + 1) * 4; \
+        int ct = (84 * 1024 - 32) / (2 * per_token + COLS * L * 4); \
+        ct = ct > 16 ? 16 : ct; \
+        const size_t smem = 2 * (size_t)(((ct * (per_token / 4)) + 3) & ~3) * 4 + (size_t)ct * COLS * L * 4; \
+        static bool opted[64] = {}; \
+        const int dev = current_device(); \
+        if (!opted[dev]) { \
+            if (cudaFuncSetAttribute(linear_scan_kernel<R, L, C, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, 84 * 1024) != cudaSuccess) \
+                return fail(HFB_ECUDA, "linear_scan: the kernel's shared memory could not be set"); \
+            opted[dev] = true; \
+        } \
+        g_launch_err = launch_pdl(linear_scan_kernel<R, L, C, DELTA>, dim3(S, H, (dv + COLS - 1) / COLS), dim3(SCAN_THREADS), smem, (cudaStream_t)s, q, q_stride, \
             k, k_stride, v, v_stride, a, a_stride, beta_logit, beta_stride, q_scale, state, (size_t)slot_stride, cu_tokens, seq_slots, n_slots, \
-            o, o_stride, H, Hq, d, dv, ct, error_word()); \
+            o, o_stride, H, Hq, d, dv, ct, (int)wide, (int)wide_state, error_word()); \
     } while (0)
-    if (d <= 32) HFB_SCAN(4, 8);
-    else if (d <= 64) HFB_SCAN(8, 8);
-    else if (d <= 128) HFB_SCAN(16, 8);
-    else if (d <= 256) HFB_SCAN(16, 16);
-    else HFB_SCAN(16, 32);
+#define HFB_SCAN(R, L, C) do { if (beta_logit) HFB_SCAN_LAUNCH(R, L, C, true); else HFB_SCAN_LAUNCH(R, L, C, false); } while (0)
+    if (d <= 32) HFB_SCAN(4, 8, 2);
+    else if (d <= 64) HFB_SCAN(8, 8, 2);
+    else if (d <= 128) HFB_SCAN(16, 8, 2);
+    else if (d <= 256) HFB_SCAN(16, 16, 2);
+    else HFB_SCAN(16, 32, 2);
+#undef HFB_SCAN_LAUNCH
 #undef HFB_SCAN
     return check_pdl_launch(g_launch_err, "linear_scan");
 }
