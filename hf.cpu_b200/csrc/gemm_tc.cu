@@ -41,8 +41,6 @@ constexpr int TILE_X = 128;            // accumulator rows (TMEM lanes)
 constexpr uint32_t X_BYTES = TILE_X * BK * 2;
 constexpr int GEMM_THREADS = 352;            // weight-tile warp, MMA warp, eight epilogue warps, activation-tile warp
 constexpr int HELPER_WARP = 10;
-constexpr int PAIR_THREADS = 224;            // pair kernel: weight-tile warp, MMA warp, four epilogue warps, activation-tile warp
-constexpr int PAIR_ACT_WARP = 6;
 
 enum { EPI_STORE = 0, EPI_ADD = 1, EPI_PARTIAL = 2, EPI_SWIGLU = 3, EPI_ROPE_KV = 4 };
 
@@ -112,15 +110,42 @@ __device__ __forceinline__ float epi_clamped_glu(const GemmParams &p, float g, f
     return __fdividef(g, 1.0f + __expf(-p.glu_alpha * g)) * (u + p.glu_offset);
 }
 
+// Eight gated pairs f = [g0, u0, g1, u1, ...].  The choice of the activation is made outside the loops: inside them the code
+// of all activations stands eight times over, and a tile's epilogue waits for its instructions (0.5B sizes, gate and up of
+// 2,048 tokens: 92 -> 67 us, and 47 us with eight epilogue warps in the pair kernel).
+__device__ __forceinline__ void epi_glu8(const GemmParams &p, const float *f, float *h)
+{
+    if (p.act == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[i] = epi_act(f[2 * i], 0) * f[2 * i + 1];
+    } else if (p.act == HFB_ACT_CLAMPED_GLU) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[i] = epi_clamped_glu(p, f[2 * i], f[2 * i + 1]);
+    } else if (p.act == HFB_ACT_GELU_TANH) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[i] = epi_act(f[2 * i], HFB_ACT_GELU_TANH) * f[2 * i + 1];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float r = fmaxf(f[2 * i], 0.f);
+            h[i] = (p.act == HFB_ACT_RELU2 ? r * r : r) * f[2 * i + 1];
+        }
+    }
+}
+
 // One chunk of 16 accumulator columns of one row: v[i] is element (xr, y0 + i) of X . Y^T.
 // `live` false: the same instructions, nothing stored (the few-token form runs its epilogue once this way while the
 // first weights are on their way, so that its code is in the instruction cache when the first tile is done: fetched
 // at that moment it waits behind the weight stream, several microseconds for a 64-token tile).
+// MANY: for a kernel whose rows are activations only (many tokens): it carries that form's code alone, and gated pairs go
+// through epi_glu8.  (The kernels of few tokens keep theirs as it is: their steps lost 1 % with either change.)
+template <bool MANY>
 __device__ __forceinline__ void epilogue_chunk(const GemmParams &p, const uint32_t *v, int xr, int y0, int split, int lane,
                                                bool live = true)
 {
-    if (!live && !p.swapped) return;
-    if (p.swapped && p.mode == EPI_SWIGLU) {
+    const bool swapped = !MANY && p.swapped;
+    if (!live && !swapped) return;
+    if (swapped && p.mode == EPI_SWIGLU) {
         // rows alternate gate, up: even lanes hold gate_i, the next lane holds up_i; out is [M, N/2].  The two lanes
         // of a pair exchange their values and share the work: of every two tokens the even lane finishes the first,
         // the odd lane the second.
@@ -144,7 +169,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams &p, const uint32
                 else ((float *)p.out)[at + (size_t)i * half_n] = h;
             }
         }
-    } else if (p.swapped) {
+    } else if (swapped) {
         // xr = output feature, y = token.  One warp per scheduler runs this, so the work per token is kept to a
         // handful of instructions: the mode is decided outside the loops, the address is a base plus i rows.
         if (xr < p.N) {
@@ -210,7 +235,9 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams &p, const uint32
                         if (y0 + i < p.N) f[i] += load_any(p.bias, p.bias_dt, y0 + i);
                 }
             }
-            if (p.act == HFB_ACT_CLAMPED_GLU) {
+            if (MANY) {
+                epi_glu8(p, f, h);
+            } else if (p.act == HFB_ACT_CLAMPED_GLU) {
 #pragma unroll
                 for (int i = 0; i < 8; i++) h[i] = epi_clamped_glu(p, f[2 * i], f[2 * i + 1]);
             } else {
@@ -435,8 +462,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                 tmem_ld16(taddr + c0, v);
                 if (two) tmem_ld16(taddr + c0 + 16, v + (BN >= 32 ? 16 : 0));
                 tmem_wait_ld();
-                epilogue_chunk(p, v, xr, ty * BN + c0, split, lane, !rehearsal);
-                if (two) epilogue_chunk(p, v + (BN >= 32 ? 16 : 0), xr, ty * BN + c0 + 16, split, lane, !rehearsal);
+                epilogue_chunk<(BN > 128)>(p, v, xr, ty * BN + c0, split, lane, !rehearsal);
+                if (two) epilogue_chunk<(BN > 128)>(p, v + (BN >= 32 ? 16 : 0), xr, ty * BN + c0 + 16, split, lane, !rehearsal);
             }
             if (rehearsal) {
                 rehearsal = false;
@@ -566,7 +593,7 @@ __device__ __forceinline__ void rope_kv_piece(const GemmParams &p, const uint32_
 }
 
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(PAIR_THREADS, 1)
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, GemmParams p, int *err)
 {
     HFB_TRACE_ENTRY(1);
@@ -585,7 +612,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     const uint32_t rank = cluster_rank();                    // 0: issues the products; 1: its peer
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
-        for (int a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 8); }   // 4 warps of 2 CTAs
+        for (int a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 16); }  // eight epilogue warps of 2 CTAs
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -605,7 +632,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     const int per_split = p.tiles_x * p.tiles_y;             // tiles_x counts tiles of 256 tokens here
     const int total_items = per_split * p.splits;
 
-    if (warp == 0 || warp == PAIR_ACT_WARP) {
+    if (warp == 0 || warp == HELPER_WARP) {
         // Two requesting threads, one per operand.  Lane 0 of warp 0 asks for this CTA's half of the weight tile and
         // arms the stage's barrier; it never waits for the kernel in front, on which the weights do not depend, so the
         // first STAGES tiles are under way long before that kernel ends.  Lane 0 of the last warp waits for it and
@@ -668,7 +695,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             if (ok && last_s >= 0) mbar_wait(empty0 + 8 * last_s, last_ph, abort_flag, err);
         }
     } else {
-        const int q = warp & 3;
+        // Two warps for each quarter of the TMEM lanes, every second 32 columns each.  (Four warps in all took 13 us a tile of
+        // 256 gated features with silu, where the products of a short inner dimension take 6.)
+        const int q = warp & 3, second = warp >= 6;
         const int row = q * 32 + lane;
         uint32_t tile_it = 0;
         bool ok = true;
@@ -692,7 +721,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 if (slot >= p.cache_slots) { atomicOr(err, HFB_ERR_SLOT); slot = -1; }
                 const float *cs = p.cos_sin + (size_t)pos * half * 2;
 #pragma unroll 1
-                for (int h0 = 0; h0 < BN; h0 += p.d) {
+                for (int piece = second; piece < BN / 64; piece += 2) {      // 32 + 32 columns, of the two halves of a head
+                    const int h0 = p.d == 64 ? piece * 64 : piece / 2 * 128, j0 = p.d == 64 ? 0 : piece % 2 * 32;
                     const int col = ty * BN + h0, head = col / p.d;
                     if (col >= p.N) break;                   // (the same for every thread)
                     __nv_bfloat16 *dst = nullptr;
@@ -701,25 +731,22 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                         else if (slot >= 0) dst = (head < p.H + p.G ? p.k_cache + ((size_t)slot * p.G + (head - p.H)) * p.d
                                                                       : p.v_cache + ((size_t)slot * p.G + (head - p.H - p.G)) * p.d);
                     }
-#pragma unroll 1
-                    for (int j0 = 0; j0 < half; j0 += 32) {
-                        uint32_t lo[32], hi[32];
-                        tmem_ld16(taddr + h0 + j0, lo); tmem_ld16(taddr + h0 + j0 + 16, lo + 16);
-                        tmem_ld16(taddr + h0 + half + j0, hi); tmem_ld16(taddr + h0 + half + j0 + 16, hi + 16);
-                        tmem_wait_ld();
-                        if (dst) rope_kv_piece(p, lo, hi, col, j0, cs, head < p.H + p.G, dst);
-                    }
+                    uint32_t lo[32], hi[32];
+                    tmem_ld16(taddr + h0 + j0, lo); tmem_ld16(taddr + h0 + j0 + 16, lo + 16);
+                    tmem_ld16(taddr + h0 + half + j0, hi); tmem_ld16(taddr + h0 + half + j0 + 16, hi + 16);
+                    tmem_wait_ld();
+                    if (dst) rope_kv_piece(p, lo, hi, col, j0, cs, head < p.H + p.G, dst);
                 }
             } else
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
+            for (int c0 = 32 * second; c0 < BN; c0 += 64) {
                 uint32_t v[32];
                 const bool two = c0 + 16 < BN;
                 tmem_ld16(taddr + c0, v);
                 if (two) tmem_ld16(taddr + c0 + 16, v + 16);
                 tmem_wait_ld();
-                epilogue_chunk(p, v, xr, ty * BN + c0, split, lane);
-                if (two) epilogue_chunk(p, v + 16, xr, ty * BN + c0 + 16, split, lane);
+                epilogue_chunk<true>(p, v, xr, ty * BN + c0, split, lane);
+                if (two) epilogue_chunk<true>(p, v + 16, xr, ty * BN + c0 + 16, split, lane);
             }
             tc_fence_before();
             __syncwarp();
@@ -912,7 +939,7 @@ static int launch_pair(const CUtensorMap &mx, const CUtensorMap &my, const GemmP
     const int pairs = items < pairs_cap ? items : pairs_cap;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(PAIR_THREADS);
+    cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
