@@ -8,7 +8,8 @@
 //   * few tokens (decode): X = weights, Y = activations (tile 128 features x BN tokens, "swapped"),
 //     so that the tensor core's 128 rows are filled by the weight matrix that has to be streamed
 //     from HBM anyway, with split-K when there are fewer weight tiles than SMs.
-// Above 128 tokens the inner dimension is split as well when the output has few tiles and K is long (mid_splits).
+// Above 128 tokens the inner dimension is cut as well when the output has few tiles: among the CTAs of a cluster
+// (gemm_tc_cluster_kernel) or, with a long K, among work items whose partial sums take a pass of their own (mid_splits).
 // Pipeline per CTA (persistent over work items): warp 0 issues TMA loads of 128-byte-swizzled K
 // blocks into a ring of shared-memory stages (the weights of the first round before the kernel in front has finished,
 // warp 10 the activations of that round as soon as it has); warp 1 issues tcgen05.mma from shared memory into one
@@ -66,6 +67,7 @@ struct GemmParams {
     __nv_bfloat16 *q_out, *k_cache, *v_cache;
     long long cache_slots;
     int n_positions, H, G, d;
+    int cluster;                       // CTAs of a cluster that share a tile's inner dimension (gemm_tc_cluster_kernel); 0: not that kernel
 };
 
 // Shared-memory operand descriptor: K-major rows of 128 bytes, 128-byte swizzle, 8-row groups 1024 bytes apart.
@@ -542,17 +544,18 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar)
                  ::"r"(bar), "h"((unsigned short)3) : "memory");
 }
 
-// The q|k|v epilogue of one head of one token (see GemmParams): `lo` and `hi` are 32 accumulator columns each, of the
+// The q|k|v epilogue of one head of one token (see GemmParams): `lo` and `hi` are W accumulator columns each, of the
 // head's first half from j0 on and of its second half from j0 on; the rotation pairs column i with column i + d/2.
+template <int W>
 __device__ __forceinline__ void rope_kv_piece(const GemmParams &p, const uint32_t *lo, const uint32_t *hi, int col, int j0,
                                               const float *cs, bool rotate, __nv_bfloat16 *dst)
 {
     const int half = p.d >> 1;
-    float bl[32], bh[32];
+    float bl[W], bh[W];
     if (p.bias) {
         const uint4 *b0 = (const uint4 *)((const __nv_bfloat16 *)p.bias + col + j0), *b1 = (const uint4 *)((const __nv_bfloat16 *)p.bias + col + half + j0);
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < W / 8; q++) {
             const uint4 x = b0[q], y = b1[q];
             const __nv_bfloat162 *hx = (const __nv_bfloat162 *)&x, *hy = (const __nv_bfloat162 *)&y;
 #pragma unroll
@@ -563,11 +566,11 @@ __device__ __forceinline__ void rope_kv_piece(const GemmParams &p, const uint32_
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < 32; i++) bl[i] = bh[i] = 0.f;
+        for (int i = 0; i < W; i++) bl[i] = bh[i] = 0.f;
     }
-    __align__(16) __nv_bfloat16 ol[32], oh[32];
+    __align__(16) __nv_bfloat16 ol[W], oh[W];
 #pragma unroll
-    for (int i = 0; i < 32; i += 2) {
+    for (int i = 0; i < W; i += 2) {
         // the separate kernels round q|k|v to bfloat16 before they rotate; the same values here
         const float a0 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(lo[i]) + bl[i]));
         const float a1 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(lo[i + 1]) + bl[i + 1]));
@@ -586,7 +589,7 @@ __device__ __forceinline__ void rope_kv_piece(const GemmParams &p, const uint32_
         }
     }
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < W / 8; q++) {
         *(uint4 *)(dst + j0 + 8 * q) = *(const uint4 *)(ol + 8 * q);
         *(uint4 *)(dst + half + j0 + 8 * q) = *(const uint4 *)(oh + 8 * q);
     }
@@ -735,7 +738,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                     tmem_ld16(taddr + h0 + j0, lo); tmem_ld16(taddr + h0 + j0 + 16, lo + 16);
                     tmem_ld16(taddr + h0 + half + j0, hi); tmem_ld16(taddr + h0 + half + j0 + 16, hi + 16);
                     tmem_wait_ld();
-                    if (dst) rope_kv_piece(p, lo, hi, col, j0, cs, head < p.H + p.G, dst);
+                    if (dst) rope_kv_piece<32>(p, lo, hi, col, j0, cs, head < p.H + p.G, dst);
                 }
             } else
 #pragma unroll 1
@@ -767,6 +770,180 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TCOLS) : "memory");
+    }
+}
+
+// ---- a few hundred tokens and few output tiles: the inner dimension cut among the CTAs of a cluster -------------
+// With M = 256 tokens and N = 896 features there are 14 tiles of 128 x 128: an SM that walks a long inner dimension alone is
+// bound by what it can take in (about 85 bytes a nanosecond), while most SMs stand idle.  Here the up to eight CTAs of a
+// cluster each multiply a slice of K into their own accumulator; then each owns an equal share of the tile's 128 rows, the
+// others put their partial sums of those rows into its shared memory (distributed shared memory: no workspace, no second
+// kernel), and after one cluster barrier it sums the slices in their order and runs the epilogue of its rows.  One tile a
+// cluster: nothing is persistent.  Roles, pipeline and bounded waits as in gemm_tc_kernel.
+// Measured: see cluster_ctas.
+constexpr int CL_BN = 128, CL_STAGES = 4, CL_ROW = CL_BN + 4;       // a row of partial sums: 16 bytes apart from the next one's banks
+constexpr uint32_t CL_Y_BYTES = CL_BN * BK * 2;
+constexpr uint32_t CL_RED_BYTES = TILE_X * CL_ROW * 4;
+constexpr uint32_t CL_SMEM = 1024 + CL_STAGES * (X_BYTES + CL_Y_BYTES) + CL_RED_BYTES + (2 * CL_STAGES + 1) * 8 + 16;
+
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// N_COLS sums of one row of the tile from column c0 on, over the live slices in their order.
+template <int N_COLS>
+__device__ __forceinline__ void cluster_row_sums(const float *red, int rows_own, int live, int row, int c0, uint32_t *v)
+{
+#pragma unroll
+    for (int c = 0; c < N_COLS; c += 4) {
+        float4 x = *(const float4 *)(red + (size_t)row * CL_ROW + c0 + c);
+        for (int s = 1; s < live; s++) {
+            const float4 y = *(const float4 *)(red + ((size_t)s * rows_own + row) * CL_ROW + c0 + c);
+            x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+        }
+        v[c] = __float_as_uint(x.x); v[c + 1] = __float_as_uint(x.y); v[c + 2] = __float_as_uint(x.z); v[c + 3] = __float_as_uint(x.w);
+    }
+}
+
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, GemmParams p, int *err)
+{
+    HFB_TRACE_ENTRY(1);
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t sx = base, sy = base + CL_STAGES * X_BYTES, sred = sy + CL_STAGES * CL_Y_BYTES;
+    const uint32_t full0 = sred + CL_RED_BYTES, empty0 = full0 + CL_STAGES * 8, tfull = empty0 + CL_STAGES * 8;
+    uint8_t *gen_base = smem_raw + (base - smem_u32(smem_raw));
+    const float *red = (const float *)(gen_base + CL_STAGES * (X_BYTES + CL_Y_BYTES));
+    volatile uint32_t *tmem_slot = (volatile uint32_t *)(gen_base + CL_STAGES * (X_BYTES + CL_Y_BYTES) + CL_RED_BYTES + (2 * CL_STAGES + 1) * 8);
+    volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < CL_STAGES; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
+        mbar_init(tfull, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32((const void *)tmem_slot)), "r"(CL_BN) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_barrier();                                           // every CTA of the cluster has started: its shared memory may be written
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    const int S = p.cluster, rank = (int)cluster_rank(), tile = blockIdx.x / S;
+    const int tx = tile % p.tiles_x, ty = tile / p.tiles_x;
+    const int kb0 = rank * p.kb_per_split, kb1 = min(kb0 + p.kb_per_split, p.kb_total);         // (the last slices may be empty)
+    const int live = (p.kb_total + p.kb_per_split - 1) / p.kb_per_split;
+    const int rows_own = TILE_X / S;
+
+    if (warp == 0 || warp == HELPER_WARP) {
+        // weights before the kernel in front has finished, activations as soon as it has (see gemm_tc_kernel)
+        const bool weights = warp == 0;
+        if (lane == 0) {
+            if (!weights) { pdl_sync(); HFB_TRACE_READY_HERE(); }
+            for (int kb = kb0, it = 0; kb < kb1; kb++, it++) {
+                const int s = it % CL_STAGES;
+                if (!mbar_wait(empty0 + 8 * s, ((it / CL_STAGES) & 1) ^ 1, abort_flag, err)) break;
+                if (weights) {
+                    mbar_arrive_expect_tx(full0 + 8 * s, X_BYTES + CL_Y_BYTES);
+                    tma_load_2d(sy + s * CL_Y_BYTES, &map_y, kb * BK, ty * CL_BN, full0 + 8 * s);
+                } else {
+                    tma_load_2d(sx + s * X_BYTES, &map_x, kb * BK, tx * TILE_X, full0 + 8 * s);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && kb0 < kb1) {
+            constexpr uint32_t idesc = instr_desc(CL_BN);
+            bool ok = true;
+            for (int kb = kb0, it = 0; kb < kb1; kb++, it++) {
+                const int s = it % CL_STAGES;
+                if (!mbar_wait(full0 + 8 * s, (it / CL_STAGES) & 1, abort_flag, err)) { ok = false; break; }
+                tc_fence_after();
+                const uint64_t dx = smem_desc(sx + s * X_BYTES), dy = smem_desc(sy + s * CL_Y_BYTES);
+#pragma unroll
+                for (int k = 0; k < BK / UMMA_K; k++)
+                    tc_mma_bf16(tmem_base, dx + 2 * k, dy + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                tc_commit(empty0 + 8 * s);
+            }
+            if (ok) {
+                tc_commit(tfull);
+                mbar_wait(tfull, 0, abort_flag, err);            // nothing of this CTA's is in flight afterwards
+            }
+        }
+    } else if (kb0 < kb1 && mbar_wait(tfull, 0, abort_flag, err)) {
+        // two warps for each quarter of the accumulator's lanes, half of the columns each: every row to the CTA that owns it
+        tc_fence_after();
+        const int q = warp & 3, row = q * 32 + lane;
+        const uint32_t dst = map_to_rank(sred + (uint32_t)((rank * rows_own + row % rows_own) * CL_ROW) * 4u, (uint32_t)(row / rows_own));
+        const int c_lo = warp >= 6 ? CL_BN / 2 : 0;
+#pragma unroll
+        for (int c0 = 0; c0 < CL_BN / 2; c0 += 32) {
+            uint32_t v[32];
+            tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + c_lo + c0, v);
+            tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + c_lo + c0 + 16, v + 16);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) st_cluster_v4(dst + (uint32_t)(c_lo + c0 + i) * 4u, v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+        tc_fence_before();
+    }
+    __syncwarp();
+    cluster_barrier();                                           // every slice's sums are where their rows' owner reads them
+
+    if (warp >= 2 && warp < HELPER_WARP && !*abort_flag) {
+        pdl_sync();                                              // nothing is written before the kernel in front has finished
+        const int t = threadIdx.x - 64;
+        if (p.mode == EPI_ROPE_KV) {
+            // pieces of 8 + 8 columns, of the two halves of a head's rotation
+            const int half = p.d >> 1, per_head = p.d >> 4;
+            for (int idx = t; idx < rows_own * (CL_BN / 16); idx += 256) {
+                const int lrow = idx % rows_own, piece = idx / rows_own;
+                const int h0 = piece / per_head * p.d, j0 = piece % per_head * 8;
+                const int xr = tx * TILE_X + rank * rows_own + lrow, col = ty * CL_BN + h0, head = col / p.d;
+                if (xr >= p.M || col >= p.N) continue;
+                int pos = p.positions[xr];
+                if (pos < 0 || pos >= p.n_positions) { atomicOr(err, HFB_ERR_POSITION); pos = 0; }
+                long long slot = p.slots ? p.slots[xr] : -1;
+                if (slot >= p.cache_slots) { atomicOr(err, HFB_ERR_SLOT); slot = -1; }
+                __nv_bfloat16 *dst = nullptr;
+                if (head < p.H) dst = p.q_out + ((size_t)xr * p.H + head) * p.d;
+                else if (slot >= 0) dst = (head < p.H + p.G ? p.k_cache + ((size_t)slot * p.G + (head - p.H)) * p.d
+                                                              : p.v_cache + ((size_t)slot * p.G + (head - p.H - p.G)) * p.d);
+                if (!dst) continue;
+                uint32_t lo[8], hi[8];
+                cluster_row_sums<8>(red, rows_own, live, lrow, h0 + j0, lo);
+                cluster_row_sums<8>(red, rows_own, live, lrow, h0 + half + j0, hi);
+                rope_kv_piece<8>(p, lo, hi, col, j0, p.cos_sin + (size_t)pos * half * 2, head < p.H + p.G, dst);
+            }
+        } else {
+            for (int idx = t; idx < rows_own * (CL_BN / 16); idx += 256) {
+                const int lrow = idx % rows_own, c0 = idx / rows_own * 16;
+                uint32_t v[16];
+                cluster_row_sums<16>(red, rows_own, live, lrow, c0, v);
+                epilogue_chunk<true>(p, v, tx * TILE_X + rank * rows_own + lrow, ty * CL_BN + c0, 0, lane);
+            }
+        }
+    }
+
+    // ---- teardown --------------------------------------------------------------------------------
+    __syncthreads();
+    if (*abort_flag && threadIdx.x == 0) {
+        // a wait ran out: give loads that are still in flight time to land before the shared memory goes away
+        for (int i = 0; i < 2000; i++) __nanosleep(1000);
+    }
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(CL_BN) : "memory");
     }
 }
 
@@ -960,6 +1137,55 @@ static int launch_pair(const CUtensorMap &mx, const CUtensorMap &my, const GemmP
     return check_pdl_launch(g_launch_err, "gemm_tc_pair");
 }
 
+static cudaLaunchConfig_t cluster_config(int tiles, int S, cudaStream_t st, cudaLaunchAttribute (&attr)[2])
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles * S);
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = CL_SMEM;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    return cfg;
+}
+
+// How many clusters of S CTAs run at once on the current device (0: none); also asks for the kernel's shared memory.
+static int cluster_slots(int S)
+{
+    static int slots[64][9];
+    static bool known[64][9];
+    static std::mutex mu;
+    const int dev = current_device();
+    std::lock_guard<std::mutex> lock(mu);
+    if (!known[dev][S]) {
+        int n = 0;
+        cudaLaunchAttribute attr[2];
+        if (cudaFuncSetAttribute(gemm_tc_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) == cudaSuccess) {
+            cudaLaunchConfig_t cfg = cluster_config(1, S, 0, attr);
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_cluster_kernel, &cfg) != cudaSuccess) n = 0;
+        }
+        cudaGetLastError();
+        slots[dev][S] = n;
+        known[dev][S] = true;
+    }
+    return slots[dev][S];
+}
+
+static int launch_cluster(const CUtensorMap &mx, const CUtensorMap &my, const GemmParams &p, cudaStream_t st)
+{
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = cluster_config(p.tiles_x * p.tiles_y, p.cluster, st, attr);
+    g_launch_err = cudaLaunchKernelEx(&cfg, gemm_tc_cluster_kernel, mx, my, p, error_word());
+    return check_pdl_launch(g_launch_err, "gemm_tc_cluster");
+}
+
 }  // namespace hfb
 
 using namespace hfb;
@@ -967,29 +1193,66 @@ using namespace hfb;
 static int pair_min_tokens() { static const int v = hfb::env_int("HFB_GEMM_PAIR", 256); return v; }     // 0: never
 static bool takes_pairs(int M) { return pair_min_tokens() > 0 && M >= pair_min_tokens() && hfb::sm_count() >= 2; }
 
-// More than 128 tokens with so few output tiles that most SMs would stand idle or wait for a few (a product with
-// few output features and a long inner dimension, at a few hundred tokens): how many ways to split the inner
-// dimension.  The cost of a choice is counted in K blocks: the rounds the busiest SM (or pair) makes over its work
-// items of 128 (or 256) tokens x 256 features, times the blocks of a slice, plus the pass over the partial sums.
-// 1: no split.
-static int mid_splits(int M, int N, int K)
+// What a product of more than 128 tokens costs the tile kernels, in nanoseconds, and (out) how many ways they split the inner
+// dimension.  With so few output tiles that most SMs would stand idle or wait for a few (a product with few output features and
+// a long inner dimension, at a few hundred tokens) K is split and the partial sums take a pass of their own; the choice of the
+// split counts K blocks: the rounds the busiest SM (or pair) makes over its work items of 128 (or 256) tokens x 256 features,
+// times the blocks of a slice, plus that pass.  A K block of a pair's tile takes about 265 ns + 0.6 ns a column, on one CTA what
+// its bytes take at 85 a nanosecond.
+static long tile_kernels_ns(int M, int N, int K, int *splits)
 {
     using namespace hfb;
     static const int on = env_int("HFB_GEMM_MID_SPLIT", 1);
-    if (!on || M <= 128) return 1;
     const bool pair = takes_pairs(M);
     const int rows = pair ? 2 * TILE_X : TILE_X, units = pair ? sm_count() / 2 : sm_count();
-    const long items = (long)((M + rows - 1) / rows) * ((N + 255) / 256);
+    const long tiles_x = (M + rows - 1) / rows, items = tiles_x * ((N + 255) / 256);
     const int kb = (K + BK - 1) / BK;
     const int per_item = 6;                             // filling the pipeline and draining the accumulator
     long best = (items + units - 1) / units * (kb + per_item);
     int best_s = 1;
-    for (int s = 2; s <= 8 && kb / s >= 32; s++) {     // shorter slices do not pay for the pass over the partial sums (measured)
+    for (int s = 2; on && s <= 8 && kb / s >= 32; s++) {     // shorter slices do not pay for the pass over the partial sums (measured)
         const long slice = (kb + s - 1) / s;
         const long cost = (items * s + units - 1) / units * (slice + per_item) + 4 + (long)s * M * N / 100000;
         if (cost < best) { best = cost; best_s = s; }
     }
-    return best_s;
+    if (splits) *splits = best_s;
+    const int widths[6] = {256, 240, 224, 208, 192, 128};
+    long ns = -1;
+    for (int i = 0; i < (best_s > 1 ? 1 : 6); i++) {
+        const long rounds = (tiles_x * ((N + widths[i] - 1) / widths[i]) * best_s + units - 1) / units;
+        const long t = rounds * ((kb + best_s - 1) / best_s) * (pair ? 265 + 6 * widths[i] / 10 : (TILE_X + widths[i]) * BK * 2 / 85);
+        if (ns < 0 || t < ns) ns = t;
+    }
+    return ns + 7000 + (best_s > 1 ? (long)best_s * M * N * 8 / 4000 : 0);
+}
+
+// The CTAs of a cluster that share a tile, for products of more than 128 tokens whose tiles of 128 x 128 all run at once; 0
+// where it is not a tenth faster than the tile kernels.  A K block takes a CTA about 360 ns (32 KB at what an SM takes in), the
+// rest 7.3 us.  Measured (us, cluster | others): 256 tokens, 896 x 4,864 11.1 | 24.4, 896 x 896 9.0 | 14.3, rotating 1,152 x 896
+// 8.3 | 12.6, 3,584 x 3,584 17.8 | 26.8, 2,048 x 5,464 17.3 | 29.3, but 3,584 x 18,944 57.5 | 44.9; 768 tokens, 896 x 4,864
+// 19.6 | 28.0, 2,048 x 5,464 43.7 | 34.7.
+static int cluster_ctas(int M, int N, int K)
+{
+    using namespace hfb;
+    static const int on = env_int("HFB_GEMM_CLUSTER", 1);
+    if (!on || M <= 128) return 0;
+    const long tiles = (long)((M + TILE_X - 1) / TILE_X) * ((N + CL_BN - 1) / CL_BN);
+    if (tiles > sm_count()) return 0;
+    const int kb = (K + BK - 1) / BK;
+    int S = 0;
+    for (int s = 8; s >= 1 && !S; s >>= 1)
+        if (kb >= 2 * s && tiles <= cluster_slots(s)) S = s;
+    if (!S) return 0;
+    return (7300 + 360L * ((kb + S - 1) / S)) * 11 / 10 < tile_kernels_ns(M, N, K, nullptr) ? S : 0;
+}
+
+// How many ways the tile kernels split the inner dimension of this product (1: they do not, or do not get it).
+static int mid_splits(int M, int N, int K)
+{
+    if (M <= 128 || cluster_ctas(M, N, K)) return 1;
+    int splits = 1;
+    tile_kernels_ns(M, N, K, &splits);
+    return splits;
 }
 
 // Common set-up of the product's tiling: fills p (sizes, tiles, maps) for `bn`.  `splits` > 1 (more than 128 tokens
@@ -1005,7 +1268,14 @@ static int plan_and_maps(const void *a, const void *w, int M, int N, int K, hfb:
     p.partial = nullptr;
     p.swapped = M <= 128;
     int rc;
-    if (p.swapped) {
+    if ((p.cluster = cluster_ctas(M, N, K)) > 0) {
+        bn = CL_BN;
+        p.tiles_x = (M + TILE_X - 1) / TILE_X;
+        p.tiles_y = (N + CL_BN - 1) / CL_BN;
+        p.kb_per_split = (p.kb_total + p.cluster - 1) / p.cluster;
+        if ((rc = tensor_map(a, M, K, TILE_X, &mx)) != HFB_OK) return rc;
+        if ((rc = tensor_map(w, N, K, CL_BN, &my)) != HFB_OK) return rc;
+    } else if (p.swapped) {
         bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
         p.tiles_x = (N + TILE_X - 1) / TILE_X;
         p.tiles_y = 1;
@@ -1044,6 +1314,7 @@ static int plan_and_maps(const void *a, const void *w, int M, int N, int K, hfb:
 static int launch_bn(int bn, const CUtensorMap &mx, const CUtensorMap &my, const hfb::GemmParams &p, cudaStream_t st)
 {
     using namespace hfb;
+    if (p.cluster) return launch_cluster(mx, my, p, st);
     if (p.pair) {
         switch (bn) {
         case 128: return launch_pair<128, 7>(mx, my, p, st);
@@ -1186,7 +1457,7 @@ extern "C" int hfb_linear_tc_act(const void *a, const void *w, void *out, int ou
     return launch_bn(bn, mx, my, p, (cudaStream_t)s);
 }
 
-// q|k|v of many tokens (256 and more: the pair kernel) with the rest of the step in the product's epilogue: bias,
+// q|k|v of many tokens (256 and more: the pair kernel; more than 128 where the cluster kernel takes the product) with the rest of the step in the product's epilogue: bias,
 // rounding to bfloat16, rotation of the query and key heads by cos_sin [n_positions, d / 2, 2] at the tokens'
 // positions, queries to q_out [M, H d], keys and values to cache slot slots[t] (null: nothing is cached).  bfloat16
 // bias and outputs, head sizes 64 and 128, the whole head rotated.  HFB_ENOTSUP, with nothing launched, where the
@@ -1196,8 +1467,8 @@ extern "C" int hfb_linear_tc_rope_kv(const void *a, const void *w, const void *b
                                      int64_t cache_slots, int M, int K, int H, int G, int d, hfb_stream s)
 {
     if (M <= 0) return HFB_OK;
-    if (!takes_pairs(M) || (d != 64 && d != 128) || H <= 0 || G <= 0 || !cos_sin || !positions || n_positions <= 0)
-        return fail(HFB_ENOTSUP, "linear_tc_rope_kv: takes 256 tokens and more, head sizes 64 and 128, a rotation table");
+    if ((!takes_pairs(M) && !cluster_ctas(M, (H + 2 * G) * d, K)) || (d != 64 && d != 128) || H <= 0 || G <= 0 || !cos_sin || !positions || n_positions <= 0)
+        return fail(HFB_ENOTSUP, "linear_tc_rope_kv: takes 256 tokens and more (129 with few tiles), head sizes 64 and 128, a rotation table");
     const int N = (H + 2 * G) * d;
     int rc = check_tc_args("linear_tc_rope_kv", a, w, q_out, M, N, K, bias);
     if (rc != HFB_OK) return rc;

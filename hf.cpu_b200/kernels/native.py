@@ -378,7 +378,7 @@ class NativeBackend:
     def linear_rope_kv(self, a, w, bias, qkv_buf, cos_sin, n_rot, positions, slots, q_out, k_cache, v_cache, H, G, d):
         self._on_gpu(a, w, bias, cos_sin, positions, slots, q_out, k_cache, v_cache)
         M, K = a.shape
-        if (self.rope_in_epilogue and M >= 256 and self._tc_ok(a, w, q_out) and q_out.dtype == torch.bfloat16
+        if (self.rope_in_epilogue and M > 128 and self._tc_ok(a, w, q_out) and q_out.dtype == torch.bfloat16
                 and k_cache.dtype == torch.bfloat16 and d in (64, 128) and n_rot == d and cos_sin is not None
                 and (bias is None or (bias.dtype == torch.bfloat16 and bias.data_ptr() % 16 == 0))):
             # many tokens: rotation and the cache write run in the product's epilogue

@@ -660,3 +660,67 @@ def test_stream_tails_of_many_tokens_are_those_of_few(dtype, M, E, S, top, split
     parts = [run(lo, min(lo + 64, M)) for lo in range(0, M, 64)]
     for i, got in enumerate(whole):
         assert torch.equal(got, torch.cat([p[i] for p in parts])), i
+
+
+# more than 128 tokens and few tiles of 128 x 128: eight, four, two and one CTA a tile, slices of unequal length, an empty last
+# slice (K of 17 and 9 pieces), ragged tokens and features, K that ends inside a piece, and one tile more than run at once
+@pytest.mark.parametrize("shape", [(129, 128, 1088), (256, 896, 4864), (255, 1152, 896), (300, 136, 200), (640, 896, 904), (130, 8, 576), (1000, 1024, 520),
+                                   (2048, 1024, 136), (256, 9472, 256), (257, 9480, 72)])
+def test_products_whose_inner_size_a_cluster_shares(shape):
+    """Exact products of bfloat16 values summed in float32: 4 sqrt(K) 2^-24 of the root sum of squares; one rounding (2^-9)
+    where the output is bfloat16."""
+    M, N, K = shape
+    b = native()
+    a, w, bias = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16), rnd(N, dtype=torch.bfloat16)
+    ref = a.double() @ w.double().T
+    bound = (K ** 0.5 + 1) * 4 * 2 ** -24 * ((a.double() ** 2) @ (w.double() ** 2).T).sqrt()
+    out = torch.full((M, N), float("nan"), device=DEV)
+    b.linear(a, w, bias, out, False)
+    want = ref + bias.double()
+    assert bool(((out.double() - want).abs() <= bound + 2 ** -23 * want.abs()).all())
+    again = torch.empty_like(out)
+    b.linear(a, w, bias, again, False)
+    assert torch.equal(out, again)
+    half = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    b.linear(a, w, bias, half, False)
+    assert torch.equal(half, out.bfloat16())
+    res = rnd(M, N, seed=3)
+    added = res.clone()
+    b.linear(a, w, None, added, True)
+    assert bool(((added.double() - res.double() - ref).abs() <= bound + 2 ** -23 * (ref.abs() + res.double().abs())).all())
+    gated = torch.empty(M, N // 2, dtype=torch.bfloat16, device=DEV)
+    b.linear_swiglu(a, (w.double() * K ** -0.5).bfloat16(), torch.empty(M, N, dtype=torch.bfloat16, device=DEV), gated)
+    z = a.double() @ (w.double() * K ** -0.5).bfloat16().double().T
+    h = torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2]
+    assert bool(((gated.double() - h).abs() <= 2 ** -8 * h.abs() + 1e-4).all())
+    b.check_device_errors()
+
+
+@pytest.mark.parametrize("M,H,G,d,K", [(129, 14, 2, 64, 896), (256, 14, 2, 64, 896), (300, 6, 2, 128, 1032), (500, 3, 1, 64, 1096), (1000, 8, 2, 128, 520)])
+def test_rotating_product_of_a_cluster(M, H, G, d, K):
+    """q|k|v with rotation and the cache write in the epilogue against the separate kernels: their sums may be cut differently, so
+    a value may round to the neighbouring bfloat16 before the rotation (2^-8 of the pair's size)."""
+    b = native()
+    back = b.backend()
+    a, w, bias = rnd(M, K, dtype=torch.bfloat16), rnd((H + 2 * G) * d, K, dtype=torch.bfloat16, scale=K ** -0.5), rnd((H + 2 * G) * d, dtype=torch.bfloat16)
+    angle = torch.rand(M + 7, d // 2, device=DEV) * 6.28
+    cs = torch.stack([angle.cos(), angle.sin()], -1).contiguous()
+    pos = torch.randperm(M, device=DEV).to(torch.int32)
+    slots = (torch.randperm(M + 16, device=DEV)[:M] - 8).to(torch.int32)           # some tokens are not cached
+    pages = (M + 31) // 16
+    got = []
+    for fused in (True, False):
+        old, back.rope_in_epilogue = back.rope_in_epilogue, fused
+        q = torch.zeros(M, H * d, dtype=torch.bfloat16, device=DEV)
+        kc, vc = (torch.zeros(pages, 16, G, d, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        try:
+            b.linear_rope_kv(a, w, bias, torch.empty(M, (H + 2 * G) * d, dtype=torch.bfloat16, device=DEV), cs, d, pos, slots, q, kc, vc, H, G, d)
+        finally:
+            back.rope_in_epilogue = old
+        got.append((q, kc, vc))
+    for x, y in zip(*got):
+        pair = y.float().unflatten(-1, (-1, d)) if x.dim() == 2 else y.float()
+        size = (pair ** 2 + pair.roll(d // 2, -1) ** 2).sqrt().view(y.shape)
+        assert bool(((x.float() - y.float()).abs() <= 2 ** -7 * size + 1e-6).all())
+        assert float((x != y).float().mean()) < 0.02
+    b.check_device_errors()
