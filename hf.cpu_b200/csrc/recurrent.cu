@@ -149,7 +149,8 @@ __global__ void conv_carry_kernel(const float *x, int splits, int x_stride, int 
 // a lane use every operand read twice.  Measured (B200, 16 heads of 128 x 128, requests of 777, 551, 324 and 97 tokens): without
 // / with the delta rule 499 / 618 us with one column a lane, scalar fma, selects for the entries behind d and copies of four
 // bytes; 229 / 319 us now; 256 threads 354 / 401 us with one column a lane, 321 / 397 us with two; 64 threads with four
-// columns 239 / 345 us.
+// columns 239 / 345 us.  Steps of 1, 8 and 64 single tokens, not overlapped: 5.2 / 5.7, 13.8 / 14.3 and 88.7 / 90.2 us; with zeros
+// written over both stages first, instead of behind d alone, 5.8 / 6.2, 14.9 / 15.7 and 94.4 / 99.9 us.
 __device__ __forceinline__ void cp_async4(float *dst, const float *src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -201,7 +202,13 @@ linear_scan_kernel(const float *q, int q_stride, const float *k, int k_stride, c
     constexpr int LC = SCAN_THREADS / L, COLS = LC * C, RS = L * (R + 4);      // columns of a block; floats of a padded row
     const int stage_floats = (ct * (3 * RS + COLS + 1) + 3) & ~3;
     float *ob = smem + 2 * stage_floats;                         // [ct][COLS * L]: every lane's pieces of o
-    for (int i = threadIdx.x; i < 2 * stage_floats; i += SCAN_THREADS) smem[i] = 0.f;        // (the entries behind d stay so)
+    if (d < R * L) {                                             // the entries behind d are zeros, and stay so
+        const int pad = R * L - d;
+        for (int idx = threadIdx.x; idx < 6 * ct * pad; idx += SCAN_THREADS) {
+            const int row = idx / pad, i = d + idx % pad;        // 3 ct rows (q, k, a) a stage
+            smem[row / (3 * ct) * stage_floats + row % (3 * ct) * RS + (i / R) * (R + 4) + i % R] = 0.f;
+        }
+    }
     pdl_wait();                                      // (a long kernel: its successor is released when the walk is done)
     const int seq = blockIdx.x, h = blockIdx.y;
     const int lcol = threadIdx.x / L, part = threadIdx.x % L, col0 = blockIdx.z * COLS;
@@ -230,7 +237,6 @@ linear_scan_kernel(const float *q, int q_stride, const float *k, int k_stride, c
             for (int r = 0; r < R; r += 2) S[c][r / 2] = pair_of(i0 + r < d ? sp[c][r] : 0.f, i0 + r + 1 < d ? sp[c][r + 1] : 0.f);
         }
     }
-    __syncthreads();                                             // the zeros are in place
 
     auto issue = [&](int c) {
         float *st = smem + (c & 1) * stage_floats;

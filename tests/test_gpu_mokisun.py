@@ -443,6 +443,44 @@ def test_recurrence_whole_in_portions_and_token_by_token(delta, geom):
     K().check_device_errors()
 
 
+# heads that fill their lanes' groups of entries (32, 64, 128, 256) and heads with zeros behind them (24, 100, 200, 300); one block of
+# columns, several, and a last one that is not full
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("geom", [(3, 3, 24, 40), (2, 1, 32, 64), (4, 2, 64, 96), (2, 2, 100, 64), (2, 1, 128, 128), (1, 1, 200, 36), (2, 1, 256, 20),
+                                  (1, 1, 300, 12)])
+def test_recurrence_reads_aligned_operands_as_others(delta, geom):
+    """Operands whose rows start on sixteen bytes come in wider copies: the same bits as slices that start anywhere (whose values the
+    test above compares with float64), a state that lies anywhere among them.  Forty tokens, three and one; one token each; all
+    behind what the earlier steps left in the slots."""
+    H, Hq, d, dv = geom
+    r = rng(H * d + dv + 7 * delta)
+    finals = []
+    steps = [[40, 3, 1], [1, 1, 1], [2, 17, 33]]
+    data = [[scan_inputs(r, n, H, Hq, d, dv) for n in lens] for lens in steps]
+    want = [plain_scan(*(f64(dev(np.concatenate([data[s][i][j] for s in range(3)]))) for j in range(5)), H, Hq, delta) for i in range(3)]
+    for pad in (0, 1):
+        store = torch.zeros(4 * H * dv * d + pad, device=DEV)
+        state = store[pad:].view(4, H, dv, d)
+        outs = [[], [], []]
+        for lens, items in zip(steps, data):
+            ops = []
+            for j, w in ((0, Hq * d), (1, Hq * d), (2, H * dv), (3, H * d)):
+                x = torch.zeros(sum(lens), w + pad, device=DEV)
+                x[:, pad:] = dev(np.concatenate([it[j].reshape(-1, w) for it in items]))
+                ops.append(x[:, pad:])
+            beta = dev(np.concatenate([it[4] for it in items])) if delta else None
+            o = torch.empty(sum(lens), H * dv, device=DEV)
+            K().linear_scan(*ops, beta, 1.0, state, step_ctx(lens, [2, 0, 3]), o, H, Hq, d, dv)
+            for i, piece in enumerate(o.split(lens)):
+                outs[i].append(piece.view(-1, H, dv))
+        finals.append([torch.cat(x) for x in outs] + [state.clone()])
+        for i in range(3):
+            assert rel(finals[-1][i], want[i]) < 2e-5
+    for x, y in zip(*finals):
+        assert torch.equal(x, y)
+    K().check_device_errors()
+
+
 @pytest.mark.parametrize("delta", [False, True])
 def test_the_state_remembers_a_token_hundreds_back(delta):
     """One early token writes a value under a key that no later token touches (later keys are orthogonal to it, decays
