@@ -724,3 +724,29 @@ def test_rotating_product_of_a_cluster(M, H, G, d, K):
         assert bool(((x.float() - y.float()).abs() <= 2 ** -7 * size + 1e-6).all())
         assert float((x != y).float().mean()) < 0.02
     b.check_device_errors()
+
+
+# few places (an expert's fit one tile of 16 or don't), many (tiles of 256), experts without any, and ids that are no expert
+@pytest.mark.parametrize("counts", [(1, 0, 0, 2), (16, 17, 0, 1, 15, 33), (0, 0, 1), (500, 12), (512, 1), (256, 257, 0, 255, 600, 1)])
+def test_places_of_the_experts(counts):
+    """Every expert's places lie one behind the other, in as few tiles as hold them, all of one size but the last."""
+    b = native()
+    E, extra = len(counts), 3
+    P = sum(counts) + extra
+    limit = b.moe_tile(P)
+    ids = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)] + [torch.tensor([E, E + 7, -1])])
+    ids = ids[torch.randperm(P, generator=torch.Generator().manual_seed(P))].to(torch.int32).to(DEV)
+    order = torch.full((P,), -5, dtype=torch.int32, device=DEV)
+    tiles = [torch.empty(b.moe_max_tiles(P, E), dtype=torch.int32, device=DEV) for _ in range(3)]
+    n_tiles = torch.empty(1, dtype=torch.int32, device=DEV)
+    b.moe_group(ids.view(P, 1), E, order, *tiles, n_tiles)
+    got = list(zip(*(t[:int(n_tiles)].tolist() for t in tiles)))
+    at, want = 0, []
+    for e, c in enumerate(counts):
+        k = -(-c // limit)
+        each = -(-c // k) if k else 0
+        want += [(e, at + p, min(each, c - p)) for p in range(0, c, max(each, 1))]
+        assert sorted(order[at:at + c].tolist()) == (ids == e).nonzero().flatten().tolist()
+        at += c
+    assert got == want and order[at:].tolist() == [-5] * extra
+    b.check_device_errors()
