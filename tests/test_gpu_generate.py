@@ -68,6 +68,35 @@ def test_bfloat16_generation_follows_plain(tiny_folders):
     assert [[c.tokens for c in comps] for comps in a] == [[c.tokens for c in comps] for comps in b]
 
 
+def test_float32_logits_are_the_same_bits_in_every_cutting(tmp_path):
+    """A prompt whole, in portions on both sides of where the products change their form, token by token, and beside other
+    requests: sums have one order, so every position's logits are the same to the bit."""
+    import hfcpu_b200
+    from hfcpu_b200.config import config_from_dict
+    cfg = dict(architectures=["Qwen2ForCausalLM"], num_hidden_layers=2, hidden_size=256, num_attention_heads=4, num_key_value_heads=2,
+               intermediate_size=1040, vocab_size=2048, max_position_embeddings=128, rms_norm_eps=1e-6, rope_theta=10000.0, tie_word_embeddings=True)
+    hfcpu_b200.write_random_model(config_from_dict(cfg), str(tmp_path), seed=5, dtype=torch.float32, std=0.1)
+    engine = hfcpu_b200.Engine(hfcpu_b200.load_model(str(tmp_path), torch.float32, "cuda:0"), block_size=16, max_tokens=256, max_requests=8)
+    ids = torch.randint(0, 2048, (90,), generator=torch.Generator().manual_seed(1)).tolist()
+
+    def logits(cuts, company=0):
+        engine.add_request("s")
+        for i in range(company):
+            engine.add_request(i)
+        rows, at = [], 0
+        for c in cuts:
+            others = [hfcpu_b200.StepEntry(i, ids[i:i + 7], [0]) for i in range(company)] if at == 0 else []
+            rows.append(engine.step([hfcpu_b200.StepEntry("s", ids[at:at + c], list(range(c)))] + others)[:c].clone())
+            at += c
+        for r in ["s"] + list(range(company)):
+            engine.finish_request(r)
+        return torch.cat(rows)
+
+    whole = logits([90])
+    for cuts, company in (([8, 82], 0), ([9, 81], 0), ([40, 3, 47], 0), ([1] * 90, 0), ([5, 85], 6)):
+        assert torch.equal(logits(cuts, company), whole), (cuts, company)
+
+
 def test_command_line_generate(tiny_folders):
     prompt = make_requests("A", [12], seed=3)["r0"]
     r = subprocess.run([sys.executable, os.path.join(ROOT, "bin", "hfb200"), "--stdin-mode", "none", "--op", "generate",

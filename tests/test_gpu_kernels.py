@@ -122,6 +122,34 @@ def test_linear_plain_forms(dtype, shape):
     assert torch.equal(out, again)
 
 
+# features and inner sizes that are cut into one, two, four and eight slices, into slices of unequal length, a size of no whole pieces;
+# few features (blocks of 32 slices of rows) and many (of 128)
+@pytest.mark.parametrize("N,K,slices", [(33, 31, 1), (38000, 200, 1), (130, 128, 2), (20000, 260, 2), (1152, 897, 8), (9728, 896, 4), (40, 1028, 8),
+                                        (896, 1184, 8), (3584, 520, 8)])
+@pytest.mark.parametrize("dtype,wdtype", [("float32", "float32"), ("float32", "bfloat16"), ("bfloat16", "float32")])
+def test_plain_product_gives_a_row_the_same_bits_in_any_company(N, K, slices, dtype, wdtype):
+    """One order of summation over k whatever the number of rows: the row counts take the streaming form, its templates, the
+    three tiles, and slices shared by a cluster as well as taken by one CTA."""
+    b = native()
+    a, w, bias = rnd(1100, K, dtype=DT[dtype]), rnd(N, K, dtype=DT[wdtype]), rnd(N)
+    counts = [1, 2, 4, 5, 8, 9, 16, 17, 64, 65, 129, 333] + ([1100] if N < 4000 else [])
+
+    def product(x, weights):
+        out = torch.full((x.shape[0], N), float("nan"), device=DEV)
+        b.linear(x, weights, bias, out, False)
+        return out
+
+    whole = product(a[:counts[-1]].contiguous(), w)
+    assert bool(whole.isfinite().all())
+    for m in counts[:-1]:
+        assert torch.equal(product(a[:m].contiguous(), w), whole[:m]), m
+    # ... and where the weights don't start on whole pieces
+    store = torch.empty(N * K + 1, dtype=w.dtype, device=DEV)
+    store[1:] = w.flatten()
+    for m in (1, 9):
+        assert torch.equal(product(a[:m].contiguous(), store[1:].view(N, K)), whole[:m])
+
+
 @pytest.mark.parametrize("geom", [(5, 1, 48, 48), (6, 3, 32, 16), (8, 8, 128, 128), (2, 2, 256, 64)])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_rope_kv_write(dtype, geom):

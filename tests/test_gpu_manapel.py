@@ -130,7 +130,7 @@ def test_router_top_k_and_softmax_over_the_chosen(dtype, geom):
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("geom", [(1, 5, 1, 72, 40, 0), (70, 5, 3, 72, 24, 56), (300, 16, 4, 256, 64, 128), (9, 2, 2, 40, 16, 8),
-                                  (200, 3, 1, 64, 200, 0)])
+                                  (200, 3, 1, 64, 200, 0), (6, 5, 2, 136, 48, 72)])
 def test_routed_experts_part(dtype, geom):
     """The feed-forward part as the engine runs it (router, grouping on the device, grouped products, weighted sum, shared
     expert) against a loop over tokens and their experts."""
