@@ -281,14 +281,22 @@ int hfb_moe_sort(const int32_t *ids, int pairs, int E, int tile, int32_t *order,
                  int32_t *tile_n, int32_t *n_tiles, hfb_stream s);
 
 /* Grouped product over the sorted places: out[dst(p), :] = act(a[src(p), :] . w[expert(p)]^T), w [E, N, K].
- * src(p) = order[p] / src_div when src_div > 0, else p; dst(p) = order[p] when scatter != 0, else p.  `a_rows`: rows of
- * `a`; `tile`: the most places a tile of the lists holds, up to 256; with 16 and less the form for steps of a few tokens
- * runs.  `rows` (bfloat16 [a_rows * src_div, K], may be null): scratch for tiles of more places with src_div > 0, whose rows
- * the tensor-core form wants one behind the other; without it such a product runs on float32 multiply-adds.  act may be HFB_ACT_GLU | HFB_ACT_CLAMPED_GLU with its constants. */
+ * src(p) = order[p] / src_div when src_div > 0, else p; dst(p) = order[p] when scatter != 0, else p.  `tile`: the most
+ * places a tile of the lists holds, up to 128; with 16 and less the form for steps of a few tokens runs.  act may be
+ * HFB_ACT_GLU | HFB_ACT_CLAMPED_GLU with its constants. */
 int hfb_moe_gemm(const void *a, int a_dt, const void *w, int w_dt, void *out, int out_dt, int act, float limit, float alpha,
-                 float offset, int a_rows, int experts, int N, int K,
+                 float offset, int N, int K,
                  const int32_t *order, int src_div, int scatter, const int32_t *tile_expert, const int32_t *tile_p0,
-                 const int32_t *tile_n, const int32_t *n_tiles, int max_tiles, int tile, void *rows, hfb_stream s);
+                 const int32_t *tile_n, const int32_t *n_tiles, int max_tiles, int tile, hfb_stream s);
+
+/* The same product for callers that say how many rows `a` has (a_rows) and how many matrices `w` (experts): tiles of more than
+ * 16 places, up to 256, then run on the 5th-generation tensor cores.  `rows` (bfloat16 [a_rows * src_div, K], 16-byte aligned):
+ * scratch for products with src_div > 0, whose rows that form wants one behind the other; without it (null) such a product
+ * runs as hfb_moe_gemm runs it. */
+int hfb_moe_gemm_rows(const void *a, int a_dt, const void *w, int w_dt, void *out, int out_dt, int act, float limit, float alpha,
+                      float offset, int a_rows, int experts, int N, int K,
+                      const int32_t *order, int src_div, int scatter, const int32_t *tile_expert, const int32_t *tile_p0,
+                      const int32_t *tile_n, const int32_t *n_tiles, int max_tiles, int tile, void *rows, hfb_stream s);
 
 /* out[t, :] = sum_j weights[t, j] * y[t * top + j, :] in float32, j in order */
 int hfb_moe_combine(const void *y, int y_dt, const float *weights, float *out, int T, int top, int N, hfb_stream s);

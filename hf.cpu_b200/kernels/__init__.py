@@ -309,11 +309,10 @@ def moe_tile(pairs: int) -> int:
     return MOE_TILE_FEW if pairs <= 512 else MOE_TILE
 
 
-
 def moe_wants_rows(pairs: int, dtype) -> bool:
     """Whether the grouped product over gathered rows runs on tiles of many places in bfloat16, whose copies want the rows of
     consecutive places one behind the other: it then asks for scratch to lay them out."""
-    return dtype == torch.bfloat16 and moe_tile(pairs) == MOE_TILE and hasattr(backend(), "lib")
+    return dtype == torch.bfloat16 and moe_tile(pairs) == MOE_TILE and getattr(backend(), "lays_out_rows", False)
 
 
 def _act(name: str) -> int:
@@ -586,9 +585,13 @@ def moe_gemm(a, w, out, act: str, order, src_div: int, scatter: bool, tile_exper
     """Grouped product over the places of :func:`moe_group`: out[dst(p)] = act(a[src(p)] @ w[expert(p)].T) with
     w [E, N, K]; src(p) = order[p] // src_div if src_div else p; dst(p) = order[p] if scatter else p.  ``glu``: the rows
     of an expert's matrix alternate gate, up, and out [.., N / 2] = act(gate) * up; act "clamped" with ``clamp`` = (limit,
-    alpha, offset) as in :func:`linear_glu`.  ``rows`` (see :func:`moe_wants_rows`): scratch [pairs, K] of ``a``'s type."""
+    alpha, offset) as in :func:`linear_glu`.  ``rows`` (see :func:`moe_wants_rows`): scratch [pairs, K] of ``a``'s type;
+    without it the call takes some from torch."""
     _need(w.dim() == 3 and a.shape[1] == w.shape[2], "moe_gemm: shape mismatch")
-    _need(rows is None or (src_div and rows.dtype == a.dtype and rows.shape == (a.shape[0] * src_div, a.shape[1])), "moe_gemm: rows are [pairs, K] of the input's type")
+    _need(rows is None or (src_div and rows.dtype == a.dtype and rows.shape == (a.shape[0] * src_div, a.shape[1])
+                            and order.numel() >= rows.shape[0]), "moe_gemm: rows are [pairs, K] of the input's type")
+    if rows is None and src_div and w.dtype == a.dtype and moe_wants_rows(int(pairs), a.dtype) and order.numel() >= a.shape[0] * src_div:
+        rows = torch.empty((a.shape[0] * src_div, a.shape[1]), dtype=a.dtype, device=a.device)
     _need((act == "clamped") == (clamp is not None) and (clamp is None or glu), "moe_gemm: the clamped form is gated and comes with its constants")
     _need(out.shape[1] == (w.shape[1] // 2 if glu else w.shape[1]) and (not glu or w.shape[1] % 2 == 0), "moe_gemm: output width mismatch")
     code = (ACT_CLAMPED_GLU if act == "clamped" else _act(act)) | (ACT_GLU if glu else 0)

@@ -43,6 +43,7 @@ def _p(t):
 
 class NativeBackend:
     name = "native"
+    lays_out_rows = True         # grouped products of many places take scratch for gathered rows (kernels.moe_wants_rows)
 
     def __init__(self):
         if not torch.cuda.is_available():
@@ -727,10 +728,10 @@ class NativeBackend:
     def moe_gemm(self, a, w, out, act, order, src_div, scatter, tile_expert, tile_p0, tile_n, n_tiles, max_tiles, tile, clamp=None, rows=None):
         self._on_gpu(a, w, out, order, tile_expert, tile_p0, tile_n, n_tiles, rows)
         consts = tuple(c_float(x) for x in (clamp or (0.0, 0.0, 0.0)))
-        self._check(self.lib.hfb_moe_gemm(_p(a), c_int(_dt(a)), _p(w), c_int(_dt(w)), _p(out), c_int(_dt(out)), c_int(act), *consts,
-                                          c_int(a.shape[0]), c_int(w.shape[0]), c_int(w.shape[1]), c_int(w.shape[2]), _p(order), c_int(src_div), c_int(1 if scatter else 0),
-                                          _p(tile_expert), _p(tile_p0), _p(tile_n), _p(n_tiles), c_int(max_tiles), c_int(tile), _p(rows),
-                                          self._stream()), "moe_gemm")
+        self._check(self.lib.hfb_moe_gemm_rows(_p(a), c_int(_dt(a)), _p(w), c_int(_dt(w)), _p(out), c_int(_dt(out)), c_int(act), *consts,
+                                               c_int(a.shape[0]), c_int(w.shape[0]), c_int(w.shape[1]), c_int(w.shape[2]), _p(order), c_int(src_div),
+                                               c_int(1 if scatter else 0), _p(tile_expert), _p(tile_p0), _p(tile_n), _p(n_tiles), c_int(max_tiles),
+                                               c_int(tile), _p(rows), self._stream()), "moe_gemm")
 
     def moe_combine(self, y, weights, out):
         self._on_gpu(y, weights, out)

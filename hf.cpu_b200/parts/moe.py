@@ -16,8 +16,8 @@ layer's input itself.
 
 Nothing comes back to the host: the router's choices are grouped by expert on the device, the experts run as one
 grouped product over the groups' tiles (launch sizes are upper bounds), and each token's choices are summed in
-the router's order, so a token's output does not depend on what else is in the step, and steps of single tokens
-replay as a graph.
+the router's order, so what its experts give a token does not depend on what else is in the step, and steps of single
+tokens replay as a graph.
 """
 from __future__ import annotations
 

@@ -656,6 +656,72 @@ def test_grouped_product(shape, act):
     b.check_device_errors()
 
 
+# tokens whose pairs are above the border of 512 in one step and below it in portions; inner sizes of one piece, several, and many
+@pytest.mark.parametrize("T,top,E,N,K", [(200, 4, 9, 136, 1032), (300, 2, 5, 64, 72), (700, 1, 3, 24, 4096), (129, 4, 32, 256, 512), (1100, 1, 2, 40, 136)])
+@pytest.mark.parametrize("act", ["none", "relu2", "silu"])
+def test_grouped_products_of_every_form_agree_to_the_bit(T, top, E, N, K, act):
+    """What a token's experts give does not depend on the number of pairs in its step, nor on whether the caller brings scratch for
+    the gathered rows, nor on which entry it calls: tcgen05, mma.sync on tiles of few places and (the entry that is not told how many
+    rows its operands have) of many add the same products in the same order.  Values over a wide range of sizes, so that an order
+    of its own would show."""
+    import ctypes
+    b = native()
+    lib, ptr = b.backend().lib, lambda t: ctypes.c_void_p(t.data_ptr() if t is not None else 0)
+    wide = lambda *shape, seed: (rnd(*shape, seed=seed) * 2.0 ** (3 * rnd(*shape, seed=seed + 1))).bfloat16()
+    a, w, hidden = wide(T, K, seed=1), wide(E, N, K, seed=3), wide(T * top, K, seed=5)
+    ids = torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(t))[:top] for t in range(T)]).to(torch.int32).to(DEV)
+    glu = act == "silu"
+
+    def lists(part, tile=0):
+        P = part.numel()
+        order = torch.empty(P, dtype=torch.int32, device=DEV)
+        tiles = [torch.empty(b.moe_max_tiles(P, E, tile), dtype=torch.int32, device=DEV) for _ in range(3)]
+        n = torch.empty(1, dtype=torch.int32, device=DEV)
+        if tile:
+            b.backend().moe_group(part, E, order, *tiles, n, tile)
+        else:
+            b.moe_group(part, E, order, *tiles, n)
+        return order, tiles, n
+
+    def by_pair(out, order):                    # rows in the order of the places -> of the (token, choice) pairs
+        y = torch.empty_like(out)
+        y[order.long()] = out
+        return y
+
+    def up(lo, hi, scratch):
+        part, P = ids[lo:hi].contiguous(), (hi - lo) * top
+        order, tiles, n = lists(part)
+        out = torch.full((P, N // 2 if glu else N), float("nan"), device=DEV)
+        rows = {"rows": torch.empty(P, K, dtype=torch.bfloat16, device=DEV)} if scratch else {}
+        b.moe_gemm(a[lo:hi].contiguous(), w, out, act, order, top, False, *tiles, n, P, glu=glu, **rows)
+        return by_pair(out, order)
+
+    def down(lo, hi):
+        part, P = ids[lo:hi].contiguous(), (hi - lo) * top
+        order, tiles, n = lists(part)
+        out = torch.full((P, N), float("nan"), device=DEV)
+        b.moe_gemm(hidden[lo * top:hi * top][order.long()].contiguous(), w, out, "none", order, 0, True, *tiles, n, P)
+        return out
+
+    whole, whole_down = up(0, T, True), down(0, T)
+    few = 512 // top
+    cuts = [(lo, min(lo + few, T)) for lo in range(0, T, few)]
+    assert T * top > 512 and bool(whole.isfinite().all())
+    assert torch.equal(up(0, T, False), whole)
+    assert torch.equal(torch.cat([up(lo, hi, False) for lo, hi in cuts]), whole)
+    assert torch.equal(torch.cat([down(lo, hi) for lo, hi in cuts]), whole_down)
+    # the entry that is not told the operands' rows: tiles of up to 128 places
+    order, tiles, n = lists(ids, 128)
+    out = torch.full_like(whole, float("nan"))
+    code = b.ACTIVATIONS[act] | (b.ACT_GLU if glu else 0)
+    call = lambda tile: lib.hfb_moe_gemm(ptr(a), 1, ptr(w), 1, ptr(out), 0, code, *[ctypes.c_float(0)] * 3, N, K, ptr(order), top, 0, *[ptr(t) for t in tiles], ptr(n),
+                                         tiles[0].numel(), tile, b.backend()._stream())
+    assert call(128) == 0
+    assert torch.equal(by_pair(out, order), whole)
+    assert call(129) == 1                       # more places than its tiles hold are refused
+    b.check_device_errors()
+
+
 # rows by columns on both sides of where steps of many tokens take four columns a thread (148 * 4,096 values), the
 # last block ragged, and a width that four does not divide
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
