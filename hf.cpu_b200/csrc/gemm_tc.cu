@@ -780,7 +780,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 // others put their partial sums of those rows into its shared memory (distributed shared memory: no workspace, no second
 // kernel), and after one cluster barrier it sums the slices in their order and runs the epilogue of its rows.  One tile a
 // cluster: nothing is persistent.  Roles, pipeline and bounded waits as in gemm_tc_kernel.
-// Measured: see cluster_ctas.
+// Measured: see choose_cut.
 constexpr int CL_BN = 128, CL_STAGES = 4, CL_ROW = CL_BN + 4;       // a row of partial sums: 16 bytes apart from the next one's banks
 constexpr uint32_t CL_Y_BYTES = CL_BN * BK * 2;
 constexpr uint32_t CL_RED_BYTES = TILE_X * CL_ROW * 4;
@@ -1155,27 +1155,26 @@ static cudaLaunchConfig_t cluster_config(int tiles, int S, cudaStream_t st, cuda
     return cfg;
 }
 
-// How many clusters of S CTAs run at once on the current device (0: none); also asks for the kernel's shared memory.
+// How many clusters of S CTAs run at once on the current device (0: it could not be told); also asks for the kernel's shared memory.
 static int cluster_slots(int S)
 {
-    static int slots[64][9];
-    static bool known[64][9];
+    static int slots[64][9];                                     // 0: not known yet
     static std::mutex mu;
     const int dev = current_device();
     std::lock_guard<std::mutex> lock(mu);
-    if (!known[dev][S]) {
+    if (slots[dev][S] == 0) {
         int n = 0;
         cudaLaunchAttribute attr[2];
-        if (cudaFuncSetAttribute(gemm_tc_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) == cudaSuccess) {
-            cudaLaunchConfig_t cfg = cluster_config(1, S, 0, attr);
-            cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_cluster_kernel, &cfg) != cudaSuccess) n = 0;
+        cudaLaunchConfig_t cfg = cluster_config(1, S, 0, attr);
+        cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(gemm_tc_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, gemm_tc_cluster_kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();                                  // (the other kernels take the product)
+            return 0;
         }
-        cudaGetLastError();
-        slots[dev][S] = n;
-        known[dev][S] = true;
+        slots[dev][S] = n > 0 ? n : -1;
     }
-    return slots[dev][S];
+    return slots[dev][S] > 0 ? slots[dev][S] : 0;
 }
 
 static int launch_cluster(const CUtensorMap &mx, const CUtensorMap &my, const GemmParams &p, cudaStream_t st)
@@ -1226,34 +1225,45 @@ static long tile_kernels_ns(int M, int N, int K, int *splits)
     return ns + 7000 + (best_s > 1 ? (long)best_s * M * N * 8 / 4000 : 0);
 }
 
-// The CTAs of a cluster that share a tile, for products of more than 128 tokens whose tiles of 128 x 128 all run at once; 0
-// where it is not a tenth faster than the tile kernels.  A K block takes a CTA about 360 ns (32 KB at what an SM takes in), the
+// How a product of more than 128 tokens is cut: the CTAs of a cluster that share a tile (0: the tile kernels take it) and the ways
+// the tile kernels split the inner dimension (1: not, or a cluster has it).
+struct Cut { int cluster, splits; };
+
+// A cluster for products whose tiles of 128 x 128 all run at once, two, four or eight CTAs to a tile, where that is a tenth faster
+// than the tile kernels.  A K block takes a CTA about 360 ns (32 KB at what an SM takes in), the
 // rest 7.3 us.  Measured (us, cluster | others): 256 tokens, 896 x 4,864 11.1 | 24.4, 896 x 896 9.0 | 14.3, rotating 1,152 x 896
 // 8.3 | 12.6, 3,584 x 3,584 17.8 | 26.8, 2,048 x 5,464 17.3 | 29.3, but 3,584 x 18,944 57.5 | 44.9; 768 tokens, 896 x 4,864
 // 19.6 | 28.0, 2,048 x 5,464 43.7 | 34.7.
-static int cluster_ctas(int M, int N, int K)
+static Cut choose_cut(int M, int N, int K)
 {
     using namespace hfb;
     static const int on = env_int("HFB_GEMM_CLUSTER", 1);
-    if (!on || M <= 128) return 0;
+    Cut c{0, 1};
+    const long ns = tile_kernels_ns(M, N, K, &c.splits);
     const long tiles = (long)((M + TILE_X - 1) / TILE_X) * ((N + CL_BN - 1) / CL_BN);
-    if (tiles > sm_count()) return 0;
+    if (!on || tiles > sm_count()) return c;
     const int kb = (K + BK - 1) / BK;
     int S = 0;
-    for (int s = 8; s >= 1 && !S; s >>= 1)
+    for (int s = 8; s >= 2 && !S; s >>= 1)
         if (kb >= 2 * s && tiles <= cluster_slots(s)) S = s;
-    if (!S) return 0;
-    return (7300 + 360L * ((kb + S - 1) / S)) * 11 / 10 < tile_kernels_ns(M, N, K, nullptr) ? S : 0;
+    if (S && (7300 + 360L * ((kb + S - 1) / S)) * 11 / 10 < ns) c = Cut{S, 1};
+    return c;
 }
 
-// How many ways the tile kernels split the inner dimension of this product (1: they do not, or do not get it).
-static int mid_splits(int M, int N, int K)
+// One product asks three to five times (for its workspace, for partial sums, for its tiling), and choosing takes up to twenty
+// divisions: a thread keeps its last answer.
+static Cut cut_of(int M, int N, int K)
 {
-    if (M <= 128 || cluster_ctas(M, N, K)) return 1;
-    int splits = 1;
-    tile_kernels_ns(M, N, K, &splits);
-    return splits;
+    if (M <= 128) return Cut{0, 1};
+    static thread_local struct { int dev, M, N, K; Cut cut; } last = {-1, 0, 0, 0, {0, 1}};
+    const int dev = hfb::current_device();
+    if (last.dev != dev || last.M != M || last.N != N || last.K != K) last = {dev, M, N, K, choose_cut(M, N, K)};
+    return last.cut;
 }
+static int cluster_ctas(int M, int N, int K) { return cut_of(M, N, K).cluster; }
+static int mid_splits(int M, int N, int K) { return cut_of(M, N, K).splits; }
+
+extern "C" int hfb_linear_tc_cluster(int M, int N, int K) { return M > 0 && N > 0 && K > 0 ? cluster_ctas(M, N, K) : 0; }
 
 // Common set-up of the product's tiling: fills p (sizes, tiles, maps) for `bn`.  `splits` > 1 (more than 128 tokens
 // only; see mid_splits) asks for that many slices of the inner dimension; the caller then sets the partial-sum mode.

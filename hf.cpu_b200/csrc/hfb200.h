@@ -58,6 +58,8 @@ int hfb_linear_plain(const void *a, int a_dt, const void *w, int w_dt, const voi
  * that kernel: `w` must be complete before the kernel in front is launched (weights are; an operand that the
  * kernel in front computes belongs in `a`).  HFB_PDL=0 in the environment turns the early start off. */
 size_t hfb_linear_tc_workspace(int M, int N, int K);
+/* How many CTAs of a cluster share a tile's inner dimension in a product of these sizes on the current device (0: none do). */
+int hfb_linear_tc_cluster(int M, int N, int K);
 int hfb_linear_tc(const void *a, const void *w, const void *bias, int bias_dt, void *out, int out_dt,
                   int accumulate, int M, int N, int K, void *workspace, size_t workspace_bytes, hfb_stream s);
 

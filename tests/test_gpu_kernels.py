@@ -756,14 +756,34 @@ def test_stream_tails_of_many_tokens_are_those_of_few(dtype, M, E, S, top, split
         assert torch.equal(got, torch.cat([p[i] for p in parts])), i
 
 
-# more than 128 tokens and few tiles of 128 x 128: eight, four, two and one CTA a tile, slices of unequal length, an empty last
-# slice (K of 17 and 9 pieces), ragged tokens and features, K that ends inside a piece, and one tile more than run at once
-@pytest.mark.parametrize("shape", [(129, 128, 1088), (256, 896, 4864), (255, 1152, 896), (300, 136, 200), (640, 896, 904), (130, 8, 576), (1000, 1024, 520),
-                                   (2048, 1024, 136), (256, 9472, 256), (257, 9480, 72)])
-def test_products_whose_inner_size_a_cluster_shares(shape):
+def cluster_of(M, N, K):
+    return native().backend().lib.hfb_linear_tc_cluster(M, N, K)
+
+
+# more than 128 tokens and few tiles of 128 x 128: eight, four and two CTAs a tile, slices of unequal length, an empty last slice (K of
+# 17 and 9 pieces), ragged tokens and features, K that ends inside a piece; then sizes that the tile kernels take (too few pieces of
+# K, or more tiles than run at once).  The largest number of tiles for a cluster size is the device's: one size is given a choice
+@pytest.mark.parametrize("shape,ctas", [((129, 128, 1088), (8,)), ((256, 896, 4864), (8,)), ((255, 1152, 896), (4,)), ((130, 8, 576), (4,)),
+                                        ((640, 896, 904), (2, 4)), ((1000, 1024, 520), (2,)), ((300, 136, 200), (0,)), ((2048, 1024, 136), (0,)),
+                                        ((256, 9472, 256), (0,)), ((257, 9480, 72), (0,))])
+def test_products_whose_inner_size_a_cluster_shares(shape, ctas):
+    assert cluster_of(*shape) in ctas
+    check_product_of_many_tokens(*shape)
+
+
+# (the inner sizes are those with which the products are worth a cluster at all)
+@pytest.mark.parametrize("ctas,K", [(8, 1032), (4, 520), (2, 520)])
+def test_products_of_as_many_tiles_as_clusters_run_at_once(ctas, K):
+    """The most tiles that a cluster size takes on this device, and the first product that it leaves to another form."""
+    M, taken = 257, [n for n in range(1, 60) if cluster_of(257, 128 * n, K) == ctas]
+    assert taken == list(range(taken[0], taken[-1] + 1)) and 3 * taken[-1] * ctas <= 148
+    for N in (128 * taken[-1], 128 * taken[-1] - 120, 128 * taken[-1] + 8):
+        check_product_of_many_tokens(M, N, K)
+
+
+def check_product_of_many_tokens(M, N, K):
     """Exact products of bfloat16 values summed in float32: 4 sqrt(K) 2^-24 of the root sum of squares; one rounding (2^-9)
     where the output is bfloat16."""
-    M, N, K = shape
     b = native()
     a, w, bias = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16), rnd(N, dtype=torch.bfloat16)
     ref = a.double() @ w.double().T
@@ -790,12 +810,15 @@ def test_products_whose_inner_size_a_cluster_shares(shape):
     b.check_device_errors()
 
 
-@pytest.mark.parametrize("M,H,G,d,K", [(129, 14, 2, 64, 896), (256, 14, 2, 64, 896), (300, 6, 2, 128, 1032), (500, 3, 1, 64, 1096), (1000, 8, 2, 128, 520)])
-def test_rotating_product_of_a_cluster(M, H, G, d, K):
+@pytest.mark.parametrize("M,H,G,d,K,ctas", [(129, 14, 2, 64, 896, 4), (256, 14, 2, 64, 896, 4), (300, 6, 2, 128, 1032, 4), (500, 3, 1, 64, 1096, 8),
+                                            (500, 16, 2, 64, 520, 2), (1000, 8, 2, 128, 520, 0)])
+def test_rotating_product_of_a_cluster(M, H, G, d, K, ctas):
     """q|k|v with rotation and the cache write in the epilogue against the separate kernels: their sums may be cut differently, so
-    a value may round to the neighbouring bfloat16 before the rotation (2^-8 of the pair's size)."""
+    a value may round to the neighbouring bfloat16 before the rotation (2^-8 of the pair's size).  The last size is the pair
+    kernel's."""
     b = native()
     back = b.backend()
+    assert cluster_of(M, (H + 2 * G) * d, K) == ctas
     a, w, bias = rnd(M, K, dtype=torch.bfloat16), rnd((H + 2 * G) * d, K, dtype=torch.bfloat16, scale=K ** -0.5), rnd((H + 2 * G) * d, dtype=torch.bfloat16)
     angle = torch.rand(M + 7, d // 2, device=DEV) * 6.28
     cs = torch.stack([angle.cos(), angle.sin()], -1).contiguous()
