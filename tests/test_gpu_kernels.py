@@ -810,6 +810,50 @@ def check_product_of_many_tokens(M, N, K):
     b.check_device_errors()
 
 
+# a cluster, one CTA a tile (129 to 255 tokens with many tiles) and pairs of CTAs; ragged tokens, features beside a tile's edge, K that
+# ends inside a piece
+@pytest.mark.parametrize("M,F,K,ctas", [(256, 448, 1032, 8), (300, 388, 520, 4), (201, 4740, 136, 0), (601, 4740, 136, 0)])
+@pytest.mark.parametrize("act", ["silu", "relu", "gelu_tanh", "relu2", "clamped"])
+def test_activations_in_the_epilogues_of_many_tokens(M, F, K, ctas, act):
+    """act(g) * u with and without a bias, into an array of its own and into columns of a wider one, in both types; act(z) alone.
+    Values around one: a sum is off by at most 4 (sqrt(K) + 1) 2^-24 of the root sum of squares of its products, a gated pair's or a
+    square's factors carry that times the other factor (below 16 here), functions and factors a few roundings of 2^-24, which the
+    fast quotient and exponential make some 2^-20, and bfloat16 outputs one rounding."""
+    b = native()
+    assert cluster_of(M, 2 * F, K) == ctas
+    a, w, bias = rnd(M, K, dtype=torch.bfloat16), rnd(2 * F, K, dtype=torch.bfloat16, scale=K ** -0.5), rnd(2 * F, dtype=torch.bfloat16)
+    clamp = (1.5, 1.7, 1.0) if act == "clamped" else None
+    fn = {"silu": torch.nn.functional.silu, "relu": torch.relu, "relu2": lambda z: z.clamp_min(0) ** 2,
+          "gelu_tanh": lambda z: torch.nn.functional.gelu(z, approximate="tanh")}.get(act)
+    z = a.double() @ w.double().T
+    slack = 32 * (K ** 0.5 + 1) * 4 * 2 ** -24 * float((a.double() ** 2).mean().sqrt())
+
+    def check(got, want):
+        assert bool(((got.double() - want).abs() <= (2 ** -8 if got.dtype == torch.bfloat16 else 2 ** -18) * want.abs() + slack).all())
+
+    for with_bias in (False, True):
+        y = z + bias.double() if with_bias else z
+        g, u = y[:, 0::2], y[:, 1::2]
+        want = g.clamp(max=1.5) * torch.sigmoid(1.7 * g.clamp(max=1.5)) * (u.clamp(-1.5, 1.5) + 1.0) if clamp else fn(g) * u
+        for dtype in (torch.bfloat16, torch.float32):
+            for wide in (0, 24):
+                store = torch.full((M, F + wide), 7.0, dtype=dtype, device=DEV)
+                out = store[:, 8:8 + F] if wide else store
+                b.linear_glu(a, w, torch.empty(M, 2 * F, dtype=dtype, device=DEV), out, act, bias=bias if with_bias else None, clamp=clamp)
+                check(out, want)
+                if wide:
+                    assert bool((store[:, :8] == 7.0).all()) and bool((store[:, 8 + F:] == 7.0).all())
+    if not clamp:
+        for dtype in (torch.bfloat16, torch.float32):
+            out = torch.full((M, 2 * F), float("nan"), dtype=dtype, device=DEV)
+            b.linear_act(a, w, out, act)
+            if act == "silu" and dtype == torch.bfloat16:        # (a pass of its own: the product is rounded before it)
+                assert rel(out, fn(z).float()) < 2 ** -7
+            else:
+                check(out, fn(z))
+    b.check_device_errors()
+
+
 @pytest.mark.parametrize("M,H,G,d,K,ctas", [(129, 14, 2, 64, 896, 4), (256, 14, 2, 64, 896, 4), (300, 6, 2, 128, 1032, 4), (500, 3, 1, 64, 1096, 8),
                                             (500, 16, 2, 64, 520, 2), (1000, 8, 2, 128, 520, 0)])
 def test_rotating_product_of_a_cluster(M, H, G, d, K, ctas):
