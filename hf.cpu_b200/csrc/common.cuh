@@ -97,6 +97,51 @@ __device__ __forceinline__ void store_any4(void *p, int dt, size_t i, float4 v)
 // Whether load_any4 / store_any4 may take the array (null: nothing will be read).
 inline bool aligned4(const void *p, int dt) { return ((uintptr_t)p & (dt == HFB_F32 ? 15 : 7)) == 0; }
 
+// Two float32 values that are worked on at once: each half rounds as an operation of its own.
+typedef unsigned long long f32pair;
+__device__ __forceinline__ f32pair pair_of(float x, float y)
+{
+    f32pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 halves(f32pair v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32pair fma2(f32pair a, f32pair b, f32pair c)
+{
+    f32pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32pair mul2(f32pair a, f32pair b)
+{
+    f32pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// The CTAs of a thread-block cluster.
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ float warp_sum(float v)
 {
 #pragma unroll

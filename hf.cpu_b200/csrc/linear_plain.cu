@@ -28,23 +28,6 @@ namespace hfb {
 constexpr int TK = 16;               // of k a stage
 constexpr int MAX_SPLITS = 8;        // CTAs of a cluster
 
-__device__ __forceinline__ unsigned long long pack2(float x, float y)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(unsigned long long v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ void fma2(unsigned long long &acc, unsigned long long a, unsigned long long b)
-{
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-
 // Four consecutive values p, those of a row from k on; zeros from K on.  VEC: K is a multiple of 4 and the rows are aligned to four values.
 template <typename T, bool VEC>
 __device__ __forceinline__ float4 load4(const T *p, int k, int K, bool live)
@@ -122,7 +105,7 @@ linear_tile_kernel(const TA *__restrict__ a, const TW *__restrict__ w, const voi
     // a thread's rows: groups of 4 (or 2) that lie BM / groups apart, its features: groups of 4, so that the lanes of a warp
     // read neighbouring 16-byte pieces
     constexpr int GM = TM >= 4 ? 4 : TM, NGM = TM / GM, NGN = TN / 4;
-    unsigned long long acc[TM][TN / 2];
+    f32pair acc[TM][TN / 2];
 #pragma unroll
     for (int i = 0; i < TM; i++)
 #pragma unroll
@@ -142,7 +125,7 @@ linear_tile_kernel(const TA *__restrict__ a, const TW *__restrict__ w, const voi
 #pragma unroll
             for (int kk = 0; kk < TK; kk++) {
                 float av[TM];
-                unsigned long long wv[TN / 2];
+                f32pair wv[TN / 2];
 #pragma unroll
                 for (int g = 0; g < NGM; g++) {
                     if constexpr (GM == 4) {
@@ -160,9 +143,9 @@ linear_tile_kernel(const TA *__restrict__ a, const TW *__restrict__ w, const voi
                 }
 #pragma unroll
                 for (int i = 0; i < TM; i++) {
-                    const unsigned long long aa = pack2(av[i], av[i]);
+                    const f32pair aa = pair_of(av[i], av[i]);
 #pragma unroll
-                    for (int j = 0; j < TN / 2; j++) fma2(acc[i][j], aa, wv[j]);
+                    for (int j = 0; j < TN / 2; j++) acc[i][j] = fma2(aa, wv[j], acc[i][j]);
                 }
             }
             if (more) put(b ^ 1);
@@ -176,7 +159,7 @@ linear_tile_kernel(const TA *__restrict__ a, const TW *__restrict__ w, const voi
             for (int i = 0; i < TM; i++)
 #pragma unroll
                 for (int j = 0; j < TN / 2; j += 2) {
-                    const float2 x = unpack2(acc[i][j]), y = unpack2(acc[i][j + 1]);
+                    const float2 x = halves(acc[i][j]), y = halves(acc[i][j + 1]);
                     float4 *t = totals + (i * (TN / 4) + j / 2) * THREADS + threadIdx.x;
                     float4 v = first ? make_float4(0.f, 0.f, 0.f, 0.f) : *t;
                     v.x += x.x; v.y += x.y; v.z += y.x; v.w += y.y;
@@ -190,9 +173,9 @@ linear_tile_kernel(const TA *__restrict__ a, const TW *__restrict__ w, const voi
 #pragma unroll
             for (int j = 0; j < TN / 2; j += 2) {
                 const float4 v = totals[(i * (TN / 4) + j / 2) * THREADS + threadIdx.x];
-                const float2 x = unpack2(acc[i][j]), y = unpack2(acc[i][j + 1]);
-                acc[i][j] = pack2(v.x + x.x, v.y + x.y);
-                acc[i][j + 1] = pack2(v.z + y.x, v.w + y.y);
+                const float2 x = halves(acc[i][j]), y = halves(acc[i][j + 1]);
+                acc[i][j] = pair_of(v.x + x.x, v.y + x.y);
+                acc[i][j + 1] = pair_of(v.z + y.x, v.w + y.y);
             }
     }
 
@@ -209,7 +192,7 @@ linear_tile_kernel(const TA *__restrict__ a, const TW *__restrict__ w, const voi
         for (int i = 0; i < TM; i++)
 #pragma unroll
             for (int j = 0; j < TN / 2; j++) {
-                const float2 v = unpack2(acc[i][j]);
+                const float2 v = halves(acc[i][j]);
                 const int gn = n0 + (j / 2) * (BN / NGN) + tx * 4 + (j & 1) * 2;
                 finish(m0 + row_of(i), gn, v.x);
                 finish(m0 + row_of(i), gn + 1, v.y);
@@ -222,25 +205,24 @@ linear_tile_kernel(const TA *__restrict__ a, const TW *__restrict__ w, const voi
     for (int i = 0; i < TM; i++)
 #pragma unroll
         for (int j = 0; j < TN / 2; j++) {
-            const float2 v = unpack2(acc[i][j]);
+            const float2 v = halves(acc[i][j]);
             *(float2 *)(sums + row_of(i) * BN + (j / 2) * (BN / NGN) + tx * 4 + (j & 1) * 2) = v;
         }
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_barrier();
     const uint32_t mine = (uint32_t)__cvta_generic_to_shared(sums);
     const int rows_each = BM / gridDim.z, first = blockIdx.z * rows_each;
     for (int e = threadIdx.x; e < rows_each * BN; e += THREADS) {
         const int r = first + e / BN, c = e % BN;
         float v = 0.f;
         for (unsigned s = 0; s < gridDim.z; s++) {
-            uint32_t at;
+            const uint32_t at = map_to_rank(mine + (uint32_t)(r * BN + c) * 4u, s);
             float x;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mine + (uint32_t)(r * BN + c) * 4u), "r"(s));
             asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(at) : "memory");
             v += x;
         }
         finish(m0 + r, n0 + c, v);
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_barrier();
 }
 
 // ---- few rows: the weights are streamed once ---------------------------------------------------------------------------

@@ -162,32 +162,6 @@ __device__ __forceinline__ void cp_async16(float *dst, const float *src)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-typedef unsigned long long f32pair;
-__device__ __forceinline__ f32pair pair_of(float x, float y)
-{
-    f32pair r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 halves(f32pair v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32pair fma2(f32pair a, f32pair b, f32pair c)
-{
-    f32pair r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32pair mul2(f32pair a, f32pair b)
-{
-    f32pair r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 constexpr int SCAN_THREADS = 128;
 
 template <int R, int L, int C, bool DELTA>

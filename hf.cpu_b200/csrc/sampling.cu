@@ -74,17 +74,9 @@ __device__ __forceinline__ void scan_row(const Row &r, F f)
 
 // ---- the cluster ----------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint32_t cluster_rank()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
 __device__ __forceinline__ uint32_t rank_addr(const void *p, uint32_t rank)
 {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
-    return r;
+    return map_to_rank(smem_addr(p), rank);
 }
 __device__ __forceinline__ float ld_rank_f32(uint32_t a)
 {
@@ -103,10 +95,6 @@ __device__ __forceinline__ unsigned long long ld_rank_u64(uint32_t a)
     unsigned long long v;
     asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
     return v;
-}
-__device__ __forceinline__ void cluster_sync_all()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Shared memory of a CTA.  `x_*` is what the CTAs of the cluster show one another, in two copies used in turn:
@@ -150,7 +138,7 @@ __device__ float cluster_sum(float v, Shared *sh, unsigned &turn)
     const float mine = block_sum(v, sh->red);
     const unsigned t = turn++ & 1;
     if (threadIdx.x == 0) sh->x_value[t] = mine;
-    cluster_sync_all();
+    cluster_barrier();
     float acc = 0.f;
     for (int rk = 0; rk < SAMPLE_CLUSTER; rk++) acc += ld_rank_f32(rank_addr(&sh->x_value[t], rk));
     return acc;
@@ -173,7 +161,7 @@ __device__ unsigned long long cluster_key(unsigned long long v, Shared *sh, unsi
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) b = LARGEST ? max(b, sh->keys[w]) : min(b, sh->keys[w]);
         sh->x_word[t] = b;
     }
-    cluster_sync_all();
+    cluster_barrier();
     unsigned long long acc = LARGEST ? 0ull : ~0ull;
     for (int rk = 0; rk < SAMPLE_CLUSTER; rk++) {
         const unsigned long long w = ld_rank_u64(rank_addr(&sh->x_word[t], rk));
@@ -259,7 +247,7 @@ __device__ unsigned long long descend(const Row &r, unsigned long long cut, floa
             for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += sh->whist[w * 256 + i];
             sh->x_hist[t][i] = s;
         }
-        cluster_sync_all();
+        cluster_barrier();
         for (int i = threadIdx.x; i < 256; i += blockDim.x) {
             float s = 0.f;
             for (int rk = 0; rk < SAMPLE_CLUSTER; rk++) s += ld_rank_f32(rank_addr(&sh->x_hist[t][i], rk));
@@ -328,7 +316,7 @@ sample_kernel(const float *logits, int V, const float *temps, const int32_t *top
     Shared *sh = &shared;
     unsigned turn = 0;
     // Nobody leaves while another CTA may still be reading its shared memory.
-    auto leave = [&]() { cluster_sync_all(); };
+    auto leave = [&]() { cluster_barrier(); };
 
     const int row = blockIdx.x / SAMPLE_CLUSTER, rank = (int)cluster_rank();
     const int share = ((V + SAMPLE_CLUSTER - 1) / SAMPLE_CLUSTER + 3) & ~3;
@@ -367,7 +355,7 @@ sample_kernel(const float *logits, int V, const float *temps, const int32_t *top
             unsigned long long k = rank_key(logit, i);
             if (k >= cut) { int at = atomicAdd(&sh->n_cand, 1); if (at < SMALL_K) found[at] = k; }
         });
-        cluster_sync_all();
+        cluster_barrier();
         if (rank != 0) return leave();
         for (int i = threadIdx.x; i < SMALL_K; i += blockDim.x) sh->cand[i] = 0;
         __syncthreads();
