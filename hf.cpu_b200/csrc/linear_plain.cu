@@ -153,19 +153,19 @@ linear_tile_kernel(const TA *__restrict__ a, const TW *__restrict__ w, const voi
             b ^= 1;
         }
         if (k0 >= k_hi) break;
-            const bool first = next == k_slice;
-            next += k_slice;
+        const bool first = next == k_slice;
+        next += k_slice;
 #pragma unroll
-            for (int i = 0; i < TM; i++)
+        for (int i = 0; i < TM; i++)
 #pragma unroll
-                for (int j = 0; j < TN / 2; j += 2) {
-                    const float2 x = halves(acc[i][j]), y = halves(acc[i][j + 1]);
-                    float4 *t = totals + (i * (TN / 4) + j / 2) * THREADS + threadIdx.x;
-                    float4 v = first ? make_float4(0.f, 0.f, 0.f, 0.f) : *t;
-                    v.x += x.x; v.y += x.y; v.z += y.x; v.w += y.y;
-                    *t = v;
-                    acc[i][j] = acc[i][j + 1] = 0ull;
-                }
+            for (int j = 0; j < TN / 2; j += 2) {
+                const float2 x = halves(acc[i][j]), y = halves(acc[i][j + 1]);
+                float4 *t = totals + (i * (TN / 4) + j / 2) * THREADS + threadIdx.x;
+                float4 v = first ? make_float4(0.f, 0.f, 0.f, 0.f) : *t;
+                v.x += x.x; v.y += x.y; v.z += y.x; v.w += y.y;
+                *t = v;
+                acc[i][j] = acc[i][j + 1] = 0ull;
+            }
     }
     if (gridDim.z == 1 && next > k_slice) {                      // the last slice's sums onto the others'
 #pragma unroll
