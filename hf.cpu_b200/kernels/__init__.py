@@ -82,6 +82,12 @@ def backend():
     return _backend
 
 
+def recorder():
+    """``record(run, tensors) -> (what run returned, recording)`` of a backend that can make a layer's launches again for layers
+    like it, or None (also while a step is profiled phase by phase)."""
+    return None if profile.enabled else getattr(backend(), "record", None)
+
+
 def set_backend(b) -> None:
     global _backend
     _backend = b

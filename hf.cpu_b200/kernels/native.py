@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
@@ -24,6 +25,56 @@ if _raw_stream is None or _current_device is None:            # (another torch: 
 
 class KernelError(RuntimeError):
     pass
+
+
+_tls = threading.local()          # .recording: the launches this thread is writing down, if any
+
+
+class Recording:
+    """The launches of one layer as they were made, for layers that differ from it in nothing but the tensors named.  A step that
+    runs kernel by kernel spends most of its time in Python choosing and checking what every layer of a model chooses alike; the
+    alike layers behind the first make the same calls with their own pointers."""
+
+    def __init__(self, backend, tensors):
+        self._backend, self._lib, self._last = backend, backend._lib, None
+        self.calls = []
+        self.ptrs = [t.data_ptr() if t is not None else 0 for t in tensors]
+        known = [p for p in self.ptrs if p]
+        self.index = {p: k for k, p in enumerate(self.ptrs) if p}
+        self.sound = len(known) == len(self.index)         # (a tensor in two places could not be told apart in another layer)
+        self.count = 0                                     # kernels the calls launch
+
+    def __getattr__(self, name):
+        fn = getattr(self._lib, name)
+
+        def call(*args):
+            self._last = fn, args
+            return fn(*args)
+        return call
+
+    def add(self, what):
+        """Keeps the call that was made last: its result has been checked, so it was a launch and no question."""
+        fn, args = self._last
+        own = [(at, self.index[a.value]) for at, a in enumerate(args) if isinstance(a, c_void_p) and a.value in self.index]
+        self.calls.append((fn, args, own, what))
+
+    def replay(self, tensors) -> bool:
+        """Makes the calls with these tensors in the places of the recorded layer's; False, with nothing launched, where one is
+        missing that was there, or aligned otherwise."""
+        ptrs = [t.data_ptr() if t is not None else 0 for t in tensors]
+        if not self.sound or any((a == 0) != (b == 0) or (a ^ b) & 255 for a, b in zip(self.ptrs, ptrs)):
+            return False
+        ptrs = [c_void_p(p) for p in ptrs]
+        for fn, args, own, what in self.calls:
+            if own:
+                args = list(args)
+                for at, k in own:
+                    args[at] = ptrs[k]
+            rc = fn(*args)
+            if rc != 0:
+                raise KernelError(f"{what}: {self._lib.hfb_last_error().decode()} (status {rc})")
+        self._backend.launches += self.count
+        return True
 
 
 F32, BF16 = 0, 1
@@ -50,7 +101,7 @@ class NativeBackend:
             raise KernelError("no CUDA device is visible: this engine has no CPU path")
         path = _build.build()
         try:
-            self.lib = ctypes.CDLL(path)
+            self._lib = ctypes.CDLL(path)
         except OSError as e:
             raise KernelError(f"the CUDA library {path} could not be loaded: {e}") from None
         self.lib.hfb_last_error.restype = ctypes.c_char_p
@@ -86,6 +137,21 @@ class NativeBackend:
         self.path = path
         self.launches = 0          # kernels launched through this binding (one per successful call)
 
+    @property
+    def lib(self):
+        return getattr(_tls, "recording", None) or self._lib
+
+    def record(self, run, tensors):
+        """``run()`` with its launches written down: (what it returned, the recording)."""
+        rec, before = Recording(self, tensors), self.launches
+        _tls.recording = rec
+        try:
+            out = run()
+        finally:
+            _tls.recording = None
+        rec.count = self.launches - before
+        return out, rec
+
     def _stream(self):
         # the raw handle of torch's current stream on the current device; asked for at every launch (a few hundred
         # a step when steps run kernel by kernel), so by the two C calls behind torch.cuda.current_stream(), which
@@ -95,6 +161,9 @@ class NativeBackend:
     def _check(self, rc: int, what: str):
         if rc != 0:
             raise KernelError(f"{what}: {self.lib.hfb_last_error().decode()} (status {rc})")
+        rec = getattr(_tls, "recording", None)
+        if rec is not None:
+            rec.add(what)
         self.launches += 1
 
     @staticmethod

@@ -108,8 +108,33 @@ class Model:
             l.block.join_outputs(l.mixer, l.ffn)
         for pos in self.positions.values():
             pos.prepare(self.plan.max_positions, self.device)
+        self._alike = self._alike_entries()
         self.bound = True
         return self
+
+    def _replay_parts(self, i: int):
+        """The parts whose kernels schedule entry ``i`` runs: its layer's, and the norm its block may write for the next."""
+        l = self.layers[self.plan.schedule[i].layer]
+        return l.norm1, l.mixer, l.norm2, l.ffn, self.layers[self.plan.schedule[i + 1].layer].norm1
+
+    def _replay_tensors(self, i: int, cache):
+        return tuple(t for p in self._replay_parts(i) for t in p.replay_tensors()) + (cache.k, cache.v)
+
+    def _alike_entries(self) -> List[Optional[int]]:
+        """For each schedule entry a number that entries share whose kernels differ in their tensors only; None for the last entry
+        and those with a part, a state or a step in front that says otherwise."""
+        numbers, out, schedule = {}, [], self.plan.schedule
+        for i, e in enumerate(schedule):
+            key = None
+            if i + 1 < len(schedule):
+                l, following = self.layers[e.layer], schedule[i + 1]
+                if (e.enter is None and following.enter is None and e.cache_of is None and l.ffn is not None and l.norm2 is not None
+                        and not l.post_norms() and l.mixer.state_spec() is None):
+                    parts = (l.block, self.layers[following.layer].block) + self._replay_parts(i)
+                    keys = tuple(p.replay_key() for p in parts)
+                    key = keys if all(k is not None for k in keys) else None
+            out.append(None if key is None else numbers.setdefault(key, len(numbers)))
+        return out
 
     def weight_bytes_per_step(self) -> int:
         """Bytes of weights one decode step reads: every schedule entry's layer and the head, once each."""
@@ -122,6 +147,7 @@ class Model:
 
     # ---- forward ------------------------------------------------------------------------
     def forward(self, ctx) -> Optional[torch.Tensor]:
+        from .. import kernels
         T = ctx.token_ids.shape[0]
         S = self.plan.streams
         x = ctx.buf("residual", (T, self.plan.hidden_size), torch.float32)
@@ -129,16 +155,26 @@ class Model:
         if S > 1:
             # the stream in S copies, a token's copies side by side, all equal to the embedding at the start
             emb, x = x, ctx.buf("residual_copies", (T, S * self.plan.hidden_size), torch.float32)
-            from .. import kernels
             with kernels.phase("glue"):
                 kernels.hc_spread(emb, x, S)
         schedule = self.plan.schedule
         for tr in self.transitions.values():
             tr.begin(ctx, x)
         xn = None                                # norm1 of the coming block, when the previous block computed it
+        record = kernels.recorder()
+        model = None                             # ((number, input, cache group), launches, output) of a layer that was written down
         for i, e in enumerate(schedule):
             layer = self.layers[e.layer]
             owner = i if e.cache_of is None else e.cache_of
+            alike = self._alike[i] if record is not None else None
+            if alike is not None:
+                cache = ctx.entry_cache(i)
+                like = alike, None if xn is None else xn.data_ptr(), cache.group
+                if model is not None and model[0] == like and model[1].replay(self._replay_tensors(i, cache)):
+                    xn = model[2]
+                    continue
+                if self._alike[i + 1] != alike or (model is not None and model[0] == like):
+                    alike = None                 # (no layer that would make the same calls follows)
             # the norm that follows this block: the next block's first, or, after the last block of a step whose
             # tokens all want their logits (a step of single tokens), the final norm
             extra = layer.post_norms()
@@ -167,9 +203,16 @@ class Model:
                 next_norm = self.final_norm if getattr(ctx, "logits_for_all", False) else None
             if layer.block.state_spec() is not None:
                 extra["block_state"] = ctx.entry_state(block_state_key(i))
-            xn = layer.block.forward(ctx, x, layer.norm1, layer.mixer, layer.norm2, layer.ffn,
-                                     ctx.entry_cache(owner), ctx.entry_state(i), e.cache_of is None,
-                                     xn_ready=xn, next_norm=next_norm, **extra)
+
+            def run():
+                return layer.block.forward(ctx, x, layer.norm1, layer.mixer, layer.norm2, layer.ffn,
+                                           ctx.entry_cache(owner), ctx.entry_state(i), e.cache_of is None,
+                                           xn_ready=xn, next_norm=next_norm, **extra)
+            if alike is None:
+                xn = run()
+            else:
+                xn, calls = record(run, self._replay_tensors(i, cache))
+                model = like, calls, xn
         M = ctx.num_logit_rows
         if M == 0:
             return None
@@ -177,7 +220,6 @@ class Model:
             xn = ctx.buf("head_xn", (M, self.plan.hidden_size), self.run_dtype)
             if S > 1:
                 # the head reads the sum of the copies
-                from .. import kernels
                 params = getattr(self.final_norm, "params", None)
                 with kernels.phase("glue"):
                     if params is not None:

@@ -287,6 +287,15 @@ class PagedAttention(OutputProduct, Mixer):
             kernels.head_gate(att, gates, out, self.H, self.dv)
         return out
 
+    def replay_key(self):
+        if type(self) is not PagedAttention or self.general or self.row_norm:
+            return None
+        return ("attention", self.E, self.H, self.G, self.d, self.mask, self.scale, id(self.rotary)) + tuple(
+            None if t is None else (t.shape, t.dtype) for t in self.replay_tensors())
+
+    def replay_tensors(self):
+        return self.w_qkv, self.b_qkv, self.w_o, self.b_o
+
     def _attend_row_norm(self, ctx, xn, cache, write_cache):
         """Heads' outputs before the gate, and the gates (None: no gate)."""
         if write_cache and not self.own_kv:

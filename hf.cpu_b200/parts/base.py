@@ -87,6 +87,15 @@ class Part:
     # engine then launches a model with such a part without that overlap
     launch_overlap_safe = True
 
+    def replay_key(self):
+        """What two parts have in common whose kernels differ in nothing but :meth:`replay_tensors`, as a hashable value; None for a
+        part that launches anything else than this engine's kernels, or reads something of the step on the host."""
+        return None
+
+    def replay_tensors(self) -> tuple:
+        """The tensors of its own this part's kernels read or write (None for one it goes without), always in the same places."""
+        return ()
+
     def tensor_specs(self) -> List[TensorSpec]:
         """The checkpoint tensors this part needs."""
         return []

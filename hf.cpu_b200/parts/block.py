@@ -33,6 +33,9 @@ class PreNormResidual(Block):
     def tensor_specs(self):
         return [TensorSpec(self.shift_tensor, (self.E,), init="half")] if self.shift_tensor else []
 
+    def replay_key(self):
+        return ("pre-norm",) if type(self) is PreNormResidual and not self.shift_tensor else None
+
     def bind(self, tensors, run_dtype, device):
         if self.shift_tensor:
             self.mu = tensors[self.shift_tensor].to(torch.float32).contiguous()

@@ -49,6 +49,14 @@ class SwiGlu(FeedForward):
             self.b_gate_up = torch.stack([tensors[self.bias_names["gate"]], tensors[self.bias_names["up"]]], 1).reshape(-1).contiguous()
             self.b_down = tensors[self.bias_names["down"]].contiguous()
 
+    def replay_key(self):
+        if type(self) is not SwiGlu:
+            return None
+        return ("swiglu", self.E, self.F, self.activation, self.clamp) + tuple(None if t is None else (t.shape, t.dtype) for t in self.replay_tensors())
+
+    def replay_tensors(self):
+        return self.w_gate_up, self.b_gate_up, self.w_down, self.b_down
+
     @property
     def operand_width(self):
         """Width of the down product's operand (what :meth:`operand` writes)."""

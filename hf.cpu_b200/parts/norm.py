@@ -34,6 +34,12 @@ class RmsNorm(Norm):
         if self.offset:
             self.weight = (self.weight.to(torch.float32) + self.offset).contiguous()
 
+    def replay_key(self):
+        return ("rms", self.size, self.eps, self.weight.dtype) if type(self) is RmsNorm and self.weight is not None else None
+
+    def replay_tensors(self):
+        return (self.weight,)
+
     def fused_args(self):
         return self.weight, self.eps
 
