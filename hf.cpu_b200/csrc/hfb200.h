@@ -96,6 +96,20 @@ int hfb_reduce_rope_kv(const float *partial, int splits, int dt, const void *bia
                        int n_rot, int n_positions, const int32_t *positions, const int32_t *slots, void *q_out,
                        void *k_cache, void *v_cache, int64_t cache_slots, int T, int H, int G, int d, hfb_stream s);
 
+/* Products of up to eight tokens, bfloat16 weights, that start at the float32 stream: with norm_w, x is float32 [M, K] and the
+ * product reads x / sqrt(mean(x^2) + eps) * norm_w; without, x is bfloat16 [M, K].  hfb_few_takes says whether the kernel has a
+ * product of these sizes (else HFB_ENOTSUP; rope: few_rope_kv has it).  few_linear: out (=|+=) product + bias.  few_glu: as hfb_linear_tc_glu.
+ * few_rope_kv: as hfb_linear_tc_rope_kv, with a bias of either type.  Like the other products they read w before they wait for
+ * the kernel in front. */
+int hfb_few_takes(int M, int N, int K, int rope);
+int hfb_few_linear(const void *x, const void *norm_w, int norm_dt, float eps, const void *w, const void *bias, int bias_dt, void *out,
+                   int out_dt, int accumulate, int M, int N, int K, hfb_stream s);
+int hfb_few_glu(const void *x, const void *norm_w, int norm_dt, float eps, const void *w, const void *bias, int bias_dt, void *out,
+                int out_dt, int64_t ldo, int M, int N, int K, int act, float limit, float alpha, float offset, hfb_stream s);
+int hfb_few_rope_kv(const void *x, const void *norm_w, int norm_dt, float eps, const void *w, const void *bias, int bias_dt,
+                    const float *cos_sin, int n_positions, const int32_t *positions, const int32_t *slots, void *q_out, void *k_cache,
+                    void *v_cache, int64_t cache_slots, int M, int K, int H, int G, int d, hfb_stream s);
+
 /* arg-max with many blocks per row (two passes; scratch of hfb_argmax2_scratch bytes). */
 size_t hfb_argmax2_scratch(int M, int V);
 int hfb_argmax2(const float *logits, int32_t *out, int M, int V, void *scratch, size_t scratch_bytes, hfb_stream s);

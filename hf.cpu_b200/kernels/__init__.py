@@ -303,6 +303,42 @@ def linear_rope_kv(a, w, bias, qkv_buf, cos_sin, n_rot, positions, slots, q_out,
     backend().linear_rope_kv(a, w, bias, qkv_buf, cos_sin, int(n_rot), positions, slots, q_out, k_cache, v_cache, H, G, d)
 
 
+FEW_TOKENS = 8               # most tokens of the products that read the stream themselves
+
+
+def few_tokens(T: int, dtype, norm, *weights, rope=None) -> bool:
+    """Whether products of ``T`` tokens with all of these matrices, behind ``norm`` = (weight, eps), are taken from the float32
+    stream on: norm, product and what follows it in one kernel each (``rope``: the matrix of :func:`few_rope_kv`; the others go to :func:`few_glu` and :func:`few_linear`)."""
+    takes = getattr(backend(), "few_takes", None)
+    return (takes is not None and T <= FEW_TOKENS and dtype == torch.bfloat16 and norm[0].data_ptr() % 16 == 0
+            and all(takes(T, w) for w in weights) and (rope is None or takes(T, rope, True)))
+
+
+def few_linear(a, norm, w, bias, out, accumulate: bool) -> None:
+    """out (=|+=) a @ w.T (+ bias) for a few tokens.  ``norm`` = (weight, eps): ``a`` is the float32 stream, and the product
+    reads ``a / sqrt(mean(a^2) + eps) * weight``."""
+    _need(a.dim() == 2 and a.shape[1] == w.shape[1] and out.shape == (a.shape[0], w.shape[0]), "few_linear: shape mismatch")
+    _need(a.dtype == (torch.float32 if norm is not None else torch.bfloat16), "few_linear: the stream is normed, bfloat16 rows are not")
+    _need(not accumulate or out.dtype == torch.float32, "few_linear: accumulation needs a float32 out")
+    backend().few_linear(a, norm, w, bias, out, bool(accumulate))
+
+
+def few_glu(a, norm, w, bias, out, activation: str, clamp=None) -> None:
+    """:func:`linear_glu` for a few tokens, the norm in front of it included (as :func:`few_linear` takes it)."""
+    _need(a.shape[1] == w.shape[1] and w.shape[0] == 2 * out.shape[1] and out.shape[0] == a.shape[0], "few_glu: shape mismatch")
+    _need(a.dtype == (torch.float32 if norm is not None else torch.bfloat16), "few_glu: the stream is normed, bfloat16 rows are not")
+    backend().few_glu(a, norm, w, bias, out, ACT_CLAMPED_GLU if activation == "clamped" else ACTIVATIONS[activation], clamp)
+
+
+def few_rope_kv(a, norm, w, bias, cos_sin, positions, slots, q_out, k_cache, v_cache, H, G, d) -> None:
+    """:func:`linear_rope_kv` for a few tokens and whole rotated heads, the norm in front of it included."""
+    _need(w.shape == ((H + 2 * G) * d, a.shape[1]) and q_out.shape == (a.shape[0], H * d), "few_rope_kv: shape mismatch")
+    _need(k_cache.shape[2:] == (G, d) and v_cache.shape == k_cache.shape and k_cache.dtype == q_out.dtype == torch.bfloat16,
+          "few_rope_kv: cache geometry mismatch")
+    _need(a.dtype == (torch.float32 if norm is not None else torch.bfloat16) and cos_sin.shape[1:] == (d // 2, 2), "few_rope_kv: input or table mismatch")
+    backend().few_rope_kv(a, norm, w, bias, cos_sin, positions, slots, q_out, k_cache, v_cache, H, G, d)
+
+
 ACT_CLAMPED_GLU = 5          # a gated pair only: see linear_glu
 ACTIVATIONS = {"silu": 0, "relu": 1, "gelu_tanh": 2, "relu2": 3, "none": 4}       # relu2: the square of relu
 ACT_GLU = 256               # added to an activation code: gated form of the grouped product

@@ -472,6 +472,37 @@ class NativeBackend:
             c_int(n_rot), c_int(npos), _p(positions), _p(slots), _p(q_out), _p(k_cache), _p(v_cache), c_int64(cache_slots),
             c_int(M), c_int(H), c_int(G), c_int(d), self._stream()), "reduce_rope_kv")
 
+    # ---- a few tokens: norm, product and what follows it in one kernel -------------------------------------
+    def few_takes(self, M, w, rope=False):
+        return (self.gemm == "tc" and w.dtype == torch.bfloat16 and w.data_ptr() % 16 == 0
+                and bool(self.lib.hfb_few_takes(c_int(M), c_int(w.shape[0]), c_int(w.shape[1]), c_int(1 if rope else 0))))
+
+    def _few_in(self, a, norm, w):
+        nw, eps = norm or (None, 0.0)
+        self._on_gpu(a, nw, w)
+        return _p(a), _p(nw), c_int(_dt(nw) if nw is not None else 0), c_float(eps), _p(w)
+
+    def few_linear(self, a, norm, w, bias, out, accumulate):
+        self._on_gpu(bias, out)
+        self._check(self.lib.hfb_few_linear(*self._few_in(a, norm, w), _p(bias), c_int(_dt(bias) if bias is not None else 0), _p(out),
+                                            c_int(_dt(out)), c_int(1 if accumulate else 0), c_int(a.shape[0]), c_int(w.shape[0]),
+                                            c_int(w.shape[1]), self._stream()), "few_linear")
+
+    def few_glu(self, a, norm, w, bias, out, act, clamp):
+        self._on_gpu(bias)
+        self._rows_on_gpu(out)
+        consts = tuple(c_float(x) for x in (clamp or (0.0, 0.0, 0.0)))
+        self._check(self.lib.hfb_few_glu(*self._few_in(a, norm, w), _p(bias), c_int(_dt(bias) if bias is not None else 0), _p(out),
+                                         c_int(_dt(out)), c_int64(out.stride(0)), c_int(a.shape[0]), c_int(w.shape[0]), c_int(w.shape[1]),
+                                         c_int(act), *consts, self._stream()), "few_glu")
+
+    def few_rope_kv(self, a, norm, w, bias, cos_sin, positions, slots, q_out, k_cache, v_cache, H, G, d):
+        self._on_gpu(bias, cos_sin, positions, slots, q_out, k_cache, v_cache)
+        self._check(self.lib.hfb_few_rope_kv(*self._few_in(a, norm, w), _p(bias), c_int(_dt(bias) if bias is not None else 0), _p(cos_sin),
+                                             c_int(cos_sin.shape[0]), _p(positions), _p(slots), _p(q_out), _p(k_cache), _p(v_cache),
+                                             c_int64(k_cache.shape[0] * k_cache.shape[1]), c_int(a.shape[0]), c_int(w.shape[1]), c_int(H),
+                                             c_int(G), c_int(d), self._stream()), "few_rope_kv")
+
     # ---- Dynamic Tanh norms, unit-rms heads, gated and routed feed-forwards --------------------------------
     def dyt(self, x, params, out, rows):
         alpha, w, b = params

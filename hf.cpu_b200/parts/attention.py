@@ -296,6 +296,22 @@ class PagedAttention(OutputProduct, Mixer):
     def replay_tensors(self):
         return self.w_qkv, self.b_qkv, self.w_o, self.b_o
 
+    def takes_stream(self, ctx, T, norm):
+        """Whether :meth:`forward_from_stream` takes a step of ``T`` tokens: the plain rotated layer, few tokens."""
+        return (not self.general and not self.row_norm and self.rotary is not None and self.rotary.n_rot == self.d and self.d in (64, 128)
+                and kernels.few_tokens(T, ctx.run_dtype, norm, self.w_o, rope=self.w_qkv))
+
+    def forward_from_stream(self, ctx, x, norm, cache, write_cache):
+        """``x += mixer(norm(x))`` with the norm in the projections' kernel (``norm`` = (weight, eps) of an RMSNorm)."""
+        T, meta = x.shape[0], ctx.group_meta(cache.group)
+        q = ctx.buf("attn_q", (T, self.QD), ctx.run_dtype)
+        with kernels.phase("qkv"):
+            kernels.few_rope_kv(x, norm, self.w_qkv, self.b_qkv, self.rotary.cos_sin, ctx.positions, meta.slots if write_cache else None, q,
+                                cache.k, cache.v, self.H, self.G, self.d)
+        att = self._softmax_attention(ctx, q, cache, meta)
+        with kernels.phase("wo"):
+            kernels.few_linear(att, None, self.w_o, self.b_o, x, True)
+
     def _attend_row_norm(self, ctx, xn, cache, write_cache):
         """Heads' outputs before the gate, and the gates (None: no gate)."""
         if write_cache and not self.own_kv:

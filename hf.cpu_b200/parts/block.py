@@ -43,8 +43,24 @@ class PreNormResidual(Block):
     def state_spec(self):
         return StateSpec((self.E,)) if self.shift_tensor else None
 
+    @staticmethod
+    def _few_tokens(ctx, x, norm1, mixer, norm2, ffn, cache, write_cache):
+        """A step of few tokens through parts that read the stream itself: the norms run in the products behind them, so that a
+        layer is five kernels instead of eight.  False (and nothing done) where a part or a norm does not know how."""
+        T = x.shape[0]
+        if T > kernels.FEW_TOKENS or not (hasattr(mixer, "takes_stream") and hasattr(ffn, "takes_stream")):
+            return False
+        n1, n2 = norm1.fused_args(), norm2.fused_args()
+        if n1 is None or n2 is None or len(n1) != 2 or len(n2) != 2 or not (mixer.takes_stream(ctx, T, n1) and ffn.takes_stream(ctx, T, n2)):
+            return False
+        mixer.forward_from_stream(ctx, x, n1, cache, write_cache)
+        ffn.forward_from_stream(ctx, x, n2)
+        return True
+
     def forward(self, ctx, x, norm1, mixer, norm2, ffn, cache, state, write_cache, xn_ready=None, next_norm=None, block_state=None,
                 next_block=None, next_block_state=None):
+        if xn_ready is None and not self.shift_tensor and ffn is not None and self._few_tokens(ctx, x, norm1, mixer, norm2, ffn, cache, write_cache):
+            return None
         if xn_ready is not None:
             xn = xn_ready                 # (from a block that knew of this block's shift, if it has one)
         elif self.shift_tensor:

@@ -85,6 +85,18 @@ class SwiGlu(FeedForward):
         with kernels.phase("down"):
             kernels.linear(h, self.w_down, self.b_down, residual, accumulate=accumulate)
 
+    def takes_stream(self, ctx, T, norm):
+        """Whether :meth:`forward_from_stream` takes a step of ``T`` tokens."""
+        return kernels.few_tokens(T, ctx.run_dtype, norm, self.w_gate_up, self.w_down)
+
+    def forward_from_stream(self, ctx, x, norm):
+        """``x += feed-forward(norm(x))`` with the norm in the front product's kernel (``norm`` = (weight, eps) of an RMSNorm)."""
+        h = ctx.buf("ffn_h", (x.shape[0], self.F), ctx.run_dtype)
+        with kernels.phase("gate_up"):
+            kernels.few_glu(x, norm, self.w_gate_up, self.b_gate_up, h, self.activation, self.clamp)
+        with kernels.phase("down"):
+            kernels.few_linear(h, None, self.w_down, self.b_down, x, True)
+
     def forward_into_norm(self, ctx, xn, y_buf, residual, post, next_norm, out):
         """residual += post(feed-forward output), the down product handed to the norm."""
         h = self._hidden(ctx, xn)
