@@ -61,6 +61,8 @@ __device__ __forceinline__ float few_act(float z, int act)
     return z / (1.0f + expf(-z));
 }
 
+template <int N> struct Count { static constexpr int value = N; };
+
 // NG groups of eight features a block.
 template <int NG>
 __global__ void __launch_bounds__(THREADS, NG <= 8 ? 3 : 2) few_kernel(const FewParams p, int *err)
@@ -97,30 +99,37 @@ __global__ void __launch_bounds__(THREADS, NG <= 8 ? 3 : 2) few_kernel(const Few
             for (int i = part * 32 + lane; i < pieces; i += per_row * 32) copy16(sx + (size_t)m * stride + i * 16, i * 8 < p.K ? src + i * 8 : src, i * 8 < p.K);
         }
     } else {
-        const int quads = pieces * 2;
-        for (int m = warp / per_row; m < p.M; m += WARPS / per_row) {
-            const float *xr = (const float *)p.x + (size_t)m * p.K;
-            float s = 0.f;
-            for (int i0 = part * 32 + lane; i0 < quads; i0 += 8 * per_row * 32) {
-                float4 v[8], nw[8];                            // sixteen reads in flight
+        // U quads of a row a lane at a time, the reads of all of them in flight
+        auto norm_rows = [&](auto count) {
+            constexpr int U = decltype(count)::value;
+            const int quads = pieces * 2, step = per_row * 32;
+            for (int m = warp / per_row; m < p.M; m += WARPS / per_row) {
+                const float *xr = (const float *)p.x + (size_t)m * p.K;
+                float s = 0.f;
+                for (int i0 = part * 32 + lane; i0 < quads; i0 += U * step) {
+                    float4 v[U], nw[U];
 #pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    const int i = i0 + u * per_row * 32;
-                    v[u] = nw[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (i * 4 < p.K) { v[u] = *(const float4 *)(xr + i * 4); nw[u] = load_any4(p.norm_w, p.norm_dt, i * 4); }
-                }
+                    for (int u = 0; u < U; u++) {
+                        const int i = i0 + u * step;
+                        v[u] = nw[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (i * 4 < p.K) { v[u] = *(const float4 *)(xr + i * 4); nw[u] = load_any4(p.norm_w, p.norm_dt, i * 4); }
+                    }
 #pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    const int i = i0 + u * per_row * 32;
-                    s += v[u].x * v[u].x + v[u].y * v[u].y + v[u].z * v[u].z + v[u].w * v[u].w;
-                    if (i < quads)
-                        store_any4(sx + (size_t)m * stride, HFB_BF16, i * 4,
-                                   make_float4(v[u].x * nw[u].x, v[u].y * nw[u].y, v[u].z * nw[u].z, v[u].w * nw[u].w));
+                    for (int u = 0; u < U; u++) {
+                        const int i = i0 + u * step;
+                        s += v[u].x * v[u].x + v[u].y * v[u].y + v[u].z * v[u].z + v[u].w * v[u].w;
+                        if (i < quads)
+                            store_any4(sx + (size_t)m * stride, HFB_BF16, i * 4,
+                                       make_float4(v[u].x * nw[u].x, v[u].y * nw[u].y, v[u].z * nw[u].z, v[u].w * nw[u].w));
+                    }
                 }
+                s = warp_sum(s);
+                if (lane == 0) ss[m * WARPS + part] = s;
             }
-            s = warp_sum(s);
-            if (lane == 0) ss[m * WARPS + part] = s;
-        }
+        };
+        if (pieces * 2 <= per_row * 32) norm_rows(Count<1>());
+        else if (pieces * 2 <= per_row * 64) norm_rows(Count<2>());
+        else norm_rows(Count<8>());
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
