@@ -340,9 +340,7 @@ class Engine:
         ctx.h_cu_tokens, ctx.h_kv_lens, ctx.h_seq_slots = cu, kv_lens, seq_slots
         ctx.max_q_len = max_q
         ctx.max_kv_len = max(kv_lens)
-        # how finely decode attention may split a request's keys: a power of two, so that few graphs exist
-        hint = max(1, ((ctx.max_kv_len + 63) // 64) // 2)
-        ctx.decode_split_hint = 1 << (min(hint, 64).bit_length() - 1)
+        ctx.decode_split_hint = kernels.decode_split_hint(ctx.max_kv_len)
         return ctx
 
     def _replay(self, ctx: StepContext) -> torch.Tensor:
