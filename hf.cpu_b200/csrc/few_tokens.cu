@@ -8,6 +8,10 @@
 // to shared memory, all of them, while that kernel still runs; what is left behind the wait is one trip to L2 for x, a few products
 // of mma.sync m16n8k16 (features on the columns, tokens on the rows, the warps share k) and one sum over the warps.  tcgen05 would
 // bring nothing: eight tokens fill an eighth of its narrowest tile, and its accumulator's trip through TMEM is latency.
+// The kernel behind is released when the wait returns: released at entry, its copies and those of the one behind it came before this
+// one's (eight steps of one token, 0.5B sizes: 5.07 against 4.63 ms).
+// Measured, a layer of the 0.5B sizes in a step of one token: 30 us with split products and their tails, 23 now; 896 x 896 and
+// 9,728 x 896, one token, where launches do not overlap: 2.7 and 7.0 us, 4.8 and 7.9 the split products without their tails.
 // Every block runs at once, one an SM: the rule (few_groups) takes matrices of which an SM holds its share in shared memory.
 #include "common.cuh"
 
@@ -25,7 +29,7 @@ struct FewParams {
     const void *norm_w; int norm_dt;   // [K] or null
     float eps;
     int mode;
-    int act;                           // FEW_GLU: the gate's activation (HFB_ACT_* code)
+    int act;                           // FEW_GLU: the gate's activation; FEW_STORE: 0 none, else the HFB_ACT_* code
     float glu_limit, glu_alpha, glu_offset;
     const void *bias; int bias_dt;     // [N] or null
     void *out; int out_dt;             // [M, N] ([M, N / 2] with FEW_GLU)
@@ -70,7 +74,6 @@ __global__ void __launch_bounds__(THREADS, NG <= 8 ? 3 : 2) few_kernel(const Few
     extern __shared__ __align__(128) unsigned char few_sm[];
     float *ss = (float *)few_sm;                               // [MAX_M][WARPS] sums of squares
     unsigned char *sm = few_sm + SS_BYTES;
-    pdl_entry();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int chunks = (p.K + FEW_CHUNK - 1) / FEW_CHUNK, pieces = chunks * (FEW_CHUNK / 8), stride = few_stride(p.K);
     constexpr int F = NG * 8;
@@ -90,7 +93,7 @@ __global__ void __launch_bounds__(THREADS, NG <= 8 ? 3 : 2) few_kernel(const Few
         const __nv_bfloat16 *src = p.w + (size_t)f * p.K;
         for (int i = lane; i < pieces; i += 32) copy16(sm + (size_t)r * stride + i * 16, i * 8 < p.K ? src + i * 8 : p.w, i * 8 < p.K);
     }
-    pdl_sync_small();
+    pdl_sync();
     // ---- x into shared memory; the normed form rounds x * w and leaves the row's factor to the finished sums
     const int per_row = p.M == 1 ? WARPS : p.M == 2 ? WARPS / 2 : p.M <= 4 ? WARPS / 4 : 1, part = warp % per_row;     // warps to a row
     if (!p.norm_w) {
@@ -220,7 +223,7 @@ __global__ void __launch_bounds__(THREADS, NG <= 8 ? 3 : 2) few_kernel(const Few
             float v = sum(m, h) * scale(m);
             if (p.bias) v += load_any(p.bias, p.bias_dt, f);
             if (p.mode == FEW_ADD) ((float *)p.out)[(size_t)m * p.ldo + f] += v;
-            else store_any(p.out, p.out_dt, (size_t)m * p.ldo + f, v);
+            else store_any(p.out, p.out_dt, (size_t)m * p.ldo + f, p.act ? few_act(v, p.act) : v);
         }
     }
 }
@@ -297,13 +300,15 @@ static int few_fill(const char *who, FewParams &p, const void *x, const void *no
 extern "C" int hfb_few_takes(int M, int N, int K, int rope) { return few_takes(M, N, K, rope != 0) ? 1 : 0; }
 
 extern "C" int hfb_few_linear(const void *x, const void *norm_w, int norm_dt, float eps, const void *w, const void *bias, int bias_dt, void *out, int out_dt,
-                              int accumulate, int M, int N, int K, hfb_stream s)
+                              int accumulate, int act, int M, int N, int K, hfb_stream s)
 {
     if (M <= 0 || N <= 0) return HFB_OK;
     FewParams p{};
     const int rc = few_fill("few_linear", p, x, norm_w, norm_dt, eps, w, bias, bias_dt, M, N, K);
     if (rc != HFB_OK) return rc;
-    if (!valid_dt(out_dt) || (accumulate && out_dt != HFB_F32)) return fail(HFB_EINVAL, "few_linear: accumulation needs a float32 output");
+    if (!valid_dt(out_dt) || (accumulate && (out_dt != HFB_F32 || act)) || act < 0 || act >= HFB_ACT_NONE)
+        return fail(HFB_EINVAL, "few_linear: accumulation needs a float32 output and no activation");
+    p.act = act;
     p.mode = accumulate ? FEW_ADD : FEW_STORE; p.out = out; p.out_dt = out_dt;
     return few_launch(p, (cudaStream_t)s);
 }

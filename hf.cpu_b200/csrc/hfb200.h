@@ -98,12 +98,13 @@ int hfb_reduce_rope_kv(const float *partial, int splits, int dt, const void *bia
 
 /* Products of up to eight tokens, bfloat16 weights, that start at the float32 stream: with norm_w, x is float32 [M, K] and the
  * product reads x / sqrt(mean(x^2) + eps) * norm_w; without, x is bfloat16 [M, K].  hfb_few_takes says whether the kernel has a
- * product of these sizes (else HFB_ENOTSUP; rope: few_rope_kv has it).  few_linear: out (=|+=) product + bias.  few_glu: as hfb_linear_tc_glu.
+ * product of these sizes (else HFB_ENOTSUP; rope: few_rope_kv has it).  few_linear: out (=|+=) act(product + bias),
+ * act 0 for none, else an HFB_ACT_* code other than silu.  few_glu: as hfb_linear_tc_glu.
  * few_rope_kv: as hfb_linear_tc_rope_kv, with a bias of either type.  Like the other products they read w before they wait for
  * the kernel in front. */
 int hfb_few_takes(int M, int N, int K, int rope);
 int hfb_few_linear(const void *x, const void *norm_w, int norm_dt, float eps, const void *w, const void *bias, int bias_dt, void *out,
-                   int out_dt, int accumulate, int M, int N, int K, hfb_stream s);
+                   int out_dt, int accumulate, int act, int M, int N, int K, hfb_stream s);
 int hfb_few_glu(const void *x, const void *norm_w, int norm_dt, float eps, const void *w, const void *bias, int bias_dt, void *out,
                 int out_dt, int64_t ldo, int M, int N, int K, int act, float limit, float alpha, float offset, hfb_stream s);
 int hfb_few_rope_kv(const void *x, const void *norm_w, int norm_dt, float eps, const void *w, const void *bias, int bias_dt,

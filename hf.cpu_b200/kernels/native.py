@@ -209,6 +209,9 @@ class NativeBackend:
         if (self.gemm == "tc" and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 8 == 0
                 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
                 and (bias is None or bias.data_ptr() % 16 == 0)):
+            if self._few(a, w):
+                self.few_linear(a, None, w, bias, out, accumulate)
+                return
             need = self.lib.hfb_linear_tc_workspace(c_int(M), c_int(N), c_int(K))
             if need:
                 self._workspace(a.device)
@@ -390,11 +393,21 @@ class NativeBackend:
             self._ws = torch.empty(64 << 20, dtype=torch.uint8, device=device)     # split-K partials never need more
         return self._ws
 
+    def _few(self, a, w):
+        """Whether the kernel of few tokens has this product (of operands :meth:`_tc_ok` has looked at).  It is the faster one
+        wherever it takes a product: one / eight tokens, us, few | split product without its tail: 896 x 896 1.9 / 2.6 | 3.3 / 3.5,
+        9,728 x 896 5.2 / 5.7 | 6.2 / 6.3, 1,024 x 2,736 2.9 / 3.5 | 3.4 / 3.5, 3,072 x 2,048 3.4 / 3.8 | 4.7 / 4.8; without
+        launches that overlap 2.7 / 3.0 | 4.8 / 4.9, 7.0 / 7.4 | 7.9 / 8.1, 4.0 / 4.3 | 5.5 / 5.6, 5.2 / 5.2 | 6.4 / 6.5."""
+        return w.numel() >= 1 << 19 and self.few_takes(a.shape[0], w)
+
     def _partials(self, a, w):
         """Split-K partial sums of a @ w.T in the workspace; returns (workspace, splits)."""
         M, K = a.shape
         N = w.shape[0]
         ws = self._workspace(a.device)
+        if self._few(a, w):                                     # one plane, the finished sums
+            self.few_linear(a, None, w, None, ws[:4 * M * N].view(torch.float32), False)
+            return ws, 1
         need = self.lib.hfb_linear_tc_partials_workspace(c_int(M), c_int(N), c_int(K))
         if need == 0 or need > ws.numel():                      # 0: above 128 rows, and not a product that is split
             return None
@@ -409,6 +422,9 @@ class NativeBackend:
         M, K = a.shape
         N = w.shape[0]
         if self._tc_ok(a, w, out):
+            if self._few(a, w):
+                self.few_glu(a, None, w, None, out, 0, None)
+                return
             self._check(self.lib.hfb_linear_tc_swiglu(_p(a), _p(w), _p(out), c_int(_dt(out)), c_int(M), c_int(N), c_int(K),
                                                       self._stream()), "linear_tc_swiglu")
             return
@@ -483,10 +499,10 @@ class NativeBackend:
         self._on_gpu(a, nw, w)
         return _p(a), _p(nw), c_int(_dt(nw) if nw is not None else 0), c_float(eps), _p(w)
 
-    def few_linear(self, a, norm, w, bias, out, accumulate):
+    def few_linear(self, a, norm, w, bias, out, accumulate, act=0):
         self._on_gpu(bias, out)
         self._check(self.lib.hfb_few_linear(*self._few_in(a, norm, w), _p(bias), c_int(_dt(bias) if bias is not None else 0), _p(out),
-                                            c_int(_dt(out)), c_int(1 if accumulate else 0), c_int(a.shape[0]), c_int(w.shape[0]),
+                                            c_int(_dt(out)), c_int(1 if accumulate else 0), c_int(act), c_int(a.shape[0]), c_int(w.shape[0]),
                                             c_int(w.shape[1]), self._stream()), "few_linear")
 
     def few_glu(self, a, norm, w, bias, out, act, clamp):
@@ -622,6 +638,9 @@ class NativeBackend:
         consts = tuple(c_float(x) for x in (clamp or (0.0, 0.0, 0.0)))
         ldo = c_int64(out.stride(0))
         if self._tc_ok(a, w, out):
+            if self._few(a, w):
+                self.few_glu(a, None, w, bias, out, act, clamp)
+                return
             M, K = a.shape
             self._check(self.lib.hfb_linear_tc_glu(_p(a), _p(w), _p(bias), b_dt, _p(out), c_int(_dt(out)), ldo, c_int(M), c_int(w.shape[0]),
                                                    c_int(K), c_int(act), *consts, self._stream()), "linear_tc_glu")
@@ -634,6 +653,9 @@ class NativeBackend:
     def linear_act(self, a, w, out, act):
         self._on_gpu(a, w, out)
         if self._tc_ok(a, w, out) and 0 < act < 4:
+            if self._few(a, w):
+                self.few_linear(a, None, w, None, out, False, act)
+                return
             M, K = a.shape
             self._check(self.lib.hfb_linear_tc_act(_p(a), _p(w), _p(out), c_int(_dt(out)), c_int(M), c_int(w.shape[0]), c_int(K),
                                                    c_int(act), self._stream()), "linear_tc_act")
