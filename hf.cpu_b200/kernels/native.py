@@ -30,6 +30,11 @@ class KernelError(RuntimeError):
 _tls = threading.local()          # .recording: the launches this thread is writing down, if any
 
 
+def _forms(tensors, ptrs):
+    """What of tensors the choice of kernels and their arguments may depend on beside the pointers themselves."""
+    return [None if t is None else (p & 255, t.shape, t.stride(), t.dtype, t.device) for t, p in zip(tensors, ptrs)]
+
+
 class Recording:
     """The launches of one layer as they were made, for layers that differ from it in nothing but the tensors named.  A step that
     runs kernel by kernel spends most of its time in Python choosing and checking what every layer of a model chooses alike; the
@@ -39,6 +44,7 @@ class Recording:
         self._backend, self._lib, self._last = backend, backend._lib, None
         self.calls = []
         self.ptrs = [t.data_ptr() if t is not None else 0 for t in tensors]
+        self.forms = _forms(tensors, self.ptrs)
         known = [p for p in self.ptrs if p]
         self.index = {p: k for k, p in enumerate(self.ptrs) if p}
         self.sound = len(known) == len(self.index)         # (a tensor in two places could not be told apart in another layer)
@@ -60,9 +66,9 @@ class Recording:
 
     def replay(self, tensors) -> bool:
         """Makes the calls with these tensors in the places of the recorded layer's; False, with nothing launched, where one is
-        missing that was there, or aligned otherwise."""
+        missing that was there, aligned otherwise, or of another shape, stride, type or device."""
         ptrs = [t.data_ptr() if t is not None else 0 for t in tensors]
-        if not self.sound or any((a == 0) != (b == 0) or (a ^ b) & 255 for a, b in zip(self.ptrs, ptrs)):
+        if not self.sound or self.forms != _forms(tensors, ptrs):
             return False
         ptrs = [c_void_p(p) for p in ptrs]
         for fn, args, own, what in self.calls:

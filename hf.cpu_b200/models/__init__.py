@@ -14,7 +14,7 @@ import torch
 
 from ..config import ModelConfig, load_config
 from ..config.base import ModelPlan
-from ..parts import make_part
+from ..parts import Part, make_part
 from ..weights import RandomSource, TensorSpec, load_tensors
 
 
@@ -36,6 +36,11 @@ class Layer:
     ffn: object
     post1: object = None
     post2: object = None
+    changes = 0                  # (no field: how many times one has been set)
+
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        vars(self)["changes"] = self.changes + 1
 
     def parts(self):
         return tuple(p for p in (self.block, self.norm1, self.mixer, self.post1, self.norm2, self.ffn, self.post2)
@@ -71,6 +76,7 @@ class Model:
         self.final_norm = make_part("norm", p.final_norm)
         self.head = make_part("head", p.head)
         self.bound = False
+        self._alike, self._watched = [], []
         self.files: List[str] = []            # the weight files this model was loaded from
 
     # ---- weights ------------------------------------------------------------------------
@@ -108,7 +114,7 @@ class Model:
             l.block.join_outputs(l.mixer, l.ffn)
         for pos in self.positions.values():
             pos.prepare(self.plan.max_positions, self.device)
-        self._alike = self._alike_entries()
+        self._look_for_alike()
         self.bound = True
         return self
 
@@ -120,20 +126,42 @@ class Model:
     def _replay_tensors(self, i: int, cache):
         return tuple(t for p in self._replay_parts(i) for t in p.replay_tensors()) + (cache.k, cache.v)
 
-    def _alike_entries(self) -> List[Optional[int]]:
-        """For each schedule entry a number that entries share whose kernels differ in their tensors only; None for the last entry
-        and those with a part, a state or a step in front that says otherwise."""
-        numbers, out, schedule = {}, [], self.plan.schedule
+    def _look_for_alike(self) -> None:
+        """``_alike``: for each schedule entry a number that entries share whose kernels differ in their tensors only; None for the
+        last entry and those with a part, a state or a step in front that says otherwise."""
+        numbers, self._alike, watched, schedule = {}, [], [], self.plan.schedule
         for i, e in enumerate(schedule):
             key = None
             if i + 1 < len(schedule):
                 l, following = self.layers[e.layer], schedule[i + 1]
+                after = self.layers[following.layer]
                 if (e.enter is None and following.enter is None and e.cache_of is None and l.ffn is not None and l.norm2 is not None
                         and not l.post_norms() and l.mixer.state_spec() is None):
-                    parts = (l.block, self.layers[following.layer].block) + self._replay_parts(i)
-                    keys = tuple(p.replay_key() for p in parts)
-                    key = keys if all(k is not None for k in keys) else None
-            out.append(None if key is None else numbers.setdefault(key, len(numbers)))
+                    parts = (l.block, after.block) + self._replay_parts(i)
+                    keys = tuple(p.replay_key() if isinstance(p, Part) else None for p in parts)
+                    if all(k is not None for k in keys):
+                        key = keys
+                        watched += [l, after, *parts]
+            self._alike.append(None if key is None else numbers.setdefault(key, len(numbers)))
+        self._watched = [(o, o.changes) for o in {id(o): o for o in watched}.values()]      # layers and parts, as they were
+        self._layers_then = list(self.layers)
+
+    def _alike_now(self) -> Optional[List[Optional[int]]]:
+        """``_alike``, None where no entries are.  What has been changed since the weights were bound (an attribute of a part, a
+        function put over one of its own, another part in its place) is alike with nothing: its own code runs."""
+        if not self._watched:
+            return None
+        if all(o.changes == n for o, n in self._watched) and len(self.layers) == len(self._layers_then) and \
+                all(a is b for a, b in zip(self.layers, self._layers_then)):
+            return self._alike
+        same = {id(o) for o, n in self._watched if o.changes == n}
+        out = []
+        for i, number in enumerate(self._alike):
+            if number is not None:
+                l, after = self.layers[self.plan.schedule[i].layer], self.layers[self.plan.schedule[i + 1].layer]
+                if not all(id(o) in same for o in (l, after, l.block, after.block) + self._replay_parts(i)):
+                    number = None
+            out.append(number)
         return out
 
     def weight_bytes_per_step(self) -> int:
@@ -162,18 +190,19 @@ class Model:
             tr.begin(ctx, x)
         xn = None                                # norm1 of the coming block, when the previous block computed it
         record = kernels.recorder()
+        alikes = self._alike_now() if record is not None else None
         model = None                             # ((number, input, cache group), launches, output) of a layer that was written down
         for i, e in enumerate(schedule):
             layer = self.layers[e.layer]
             owner = i if e.cache_of is None else e.cache_of
-            alike = self._alike[i] if record is not None else None
+            alike = alikes[i] if alikes is not None else None
             if alike is not None:
                 cache = ctx.entry_cache(i)
                 like = alike, None if xn is None else xn.data_ptr(), cache.group
                 if model is not None and model[0] == like and model[1].replay(self._replay_tensors(i, cache)):
                     xn = model[2]
                     continue
-                if self._alike[i + 1] != alike or (model is not None and model[0] == like):
+                if alikes[i + 1] != alike or (model is not None and model[0] == like):
                     alike = None                 # (no layer that would make the same calls follows)
             # the norm that follows this block: the next block's first, or, after the last block of a step whose
             # tokens all want their logits (a step of single tokens), the final norm
@@ -212,7 +241,7 @@ class Model:
                 xn = run()
             else:
                 xn, calls = record(run, self._replay_tensors(i, cache))
-                model = like, calls, xn
+                model = (like, calls, xn) if calls is not None else None
         M = ctx.num_logit_rows
         if M == 0:
             return None

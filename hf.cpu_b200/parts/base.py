@@ -86,14 +86,26 @@ class Part:
     # False for a part whose kernels have not been cleared to start before the kernel in front of them has finished; the
     # engine then launches a model with such a part without that overlap
     launch_overlap_safe = True
+    # how many times an attribute has been set or taken away: what was found out about a part holds while this stays
+    changes = 0
+
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        vars(self)["changes"] = self.changes + 1
+
+    def __delattr__(self, name):
+        super().__delattr__(name)
+        vars(self)["changes"] = self.changes + 1
 
     def replay_key(self):
         """What two parts have in common whose kernels differ in nothing but :meth:`replay_tensors`, as a hashable value; None for a
-        part that launches anything else than this engine's kernels, or reads something of the step on the host."""
+        part that launches anything else than this engine's kernels, or reads something of the step on the host.  Asked for once, when
+        the weights are bound: a part that is changed afterwards runs its own code again."""
         return None
 
     def replay_tensors(self) -> tuple:
-        """The tensors of its own this part's kernels read or write (None for one it goes without), always in the same places."""
+        """The tensors of its own this part's kernels read or write (None for one it goes without), always in the same places.  The
+        kernels are given each by its first element."""
         return ()
 
     def tensor_specs(self) -> List[TensorSpec]:

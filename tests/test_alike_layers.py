@@ -1,0 +1,196 @@
+"""Layers whose launches are made again from another layer's recording: whatever has been changed since the weights were bound runs
+its own code.  On the CPU, with a stand-in that writes down its calls as the CUDA backend does, and the CUDA backend's recording
+itself against a stand-in library."""
+import ctypes
+
+import pytest
+import torch
+
+from emu_backend import EmuBackend
+
+CFG = dict(architectures=["Qwen2ForCausalLM"], num_hidden_layers=6, hidden_size=64, num_attention_heads=4, num_key_value_heads=2,
+           intermediate_size=96, vocab_size=200, max_position_embeddings=128, rms_norm_eps=1e-6, rope_theta=1e4, tie_word_embeddings=False)
+
+
+class RecordingEmu(EmuBackend):
+    """The stand-in with a recorder: a recording makes the calls again with other tensors in the places of the recorded ones."""
+
+    def __init__(self):
+        self.log, self.replayed = None, 0
+
+    def __getattribute__(self, name):
+        fn = object.__getattribute__(self, name)
+        if name.startswith("_") or name == "record" or not callable(fn):
+            return fn
+
+        def call(*args, **kw):
+            if self.log is not None:
+                self.log.append((fn, args, kw))
+            saved, self.log = self.log, None               # (a call that makes others is one call)
+            try:
+                return fn(*args, **kw)
+            finally:
+                self.log = saved
+        return call
+
+    def record(self, run, tensors):
+        self.log = []
+        out = run()
+        calls, self.log = self.log, None
+        owner = self
+
+        class Recording:
+            def replay(self, others):
+                assert len(others) == len(tensors)
+                ptrs = {t.data_ptr(): o for t, o in zip(tensors, others) if t is not None}
+
+                def swap(a):
+                    return ptrs.get(a.data_ptr(), a) if isinstance(a, torch.Tensor) else a
+                for fn, args, kw in calls:
+                    fn(*[swap(a) for a in args], **{k: swap(a) for k, a in kw.items()})
+                owner.replayed += 1
+                return True
+        return out, Recording()
+
+
+@pytest.fixture
+def emu():
+    from hfcpu_b200 import kernels
+    old, b = kernels._backend, RecordingEmu()
+    kernels.set_backend(b)
+    yield b
+    kernels.set_backend(old)
+
+
+def _model():
+    from hfcpu_b200.config import config_from_dict
+    from hfcpu_b200.models import random_model
+    return random_model(config_from_dict(CFG), seed=5, dtype=torch.float32, device="cpu", std=0.2)
+
+
+def _steps(model, record=True):
+    """Logits of a portion of 12 tokens and two single tokens."""
+    import hfcpu_b200
+    from hfcpu_b200 import kernels
+    eng, saved = hfcpu_b200.Engine(model, block_size=16, max_tokens=256, max_requests=2), kernels.recorder
+    eng.add_request("a")
+    if not record:
+        kernels.recorder = lambda: None
+    try:
+        return torch.cat([eng.step([hfcpu_b200.StepEntry("a", [(7 * i + n) % 200 for i in range(n)], [n - 1])]).clone() for n in (12, 1, 1)])
+    finally:
+        kernels.recorder = saved
+
+
+def test_alike_layers_are_made_again(emu):
+    model = _model()
+    assert model._alike == [0] * 5 + [None]
+    want = _steps(model, record=False)
+    assert emu.replayed == 0
+    assert torch.equal(_steps(model), want)
+    assert emu.replayed == 3 * 3                       # three steps; of five alike layers the first gets its input otherwise, the second is written down
+
+
+def _other_ffn(model):
+    from hfcpu_b200.parts import make_part
+    part = make_part("ffn", type(model.plan.layers[0].ffn)("swiglu", dict(model.plan.layers[0].ffn.args, activation="relu")))
+    part.w_gate_up, part.w_down = model.layers[2].ffn.w_gate_up, model.layers[2].ffn.w_down
+    return part
+
+
+def _new_layer(model):
+    from hfcpu_b200.models import Layer
+    l = model.layers[3]
+    return Layer(l.block, l.norm1, l.mixer, l.norm2, _other_ffn(model))
+
+
+CHANGES = {
+    "a part's method": lambda m: setattr(m.layers[2].mixer, "_attend", lambda ctx, xn, cache, write: torch.ones_like(xn)),
+    "the feed-forward's method": lambda m: setattr(m.layers[3].ffn, "_hidden", lambda ctx, xn: torch.ones(xn.shape[0], 96)),
+    "a block's forward": lambda m: setattr(m.layers[2].block, "forward", lambda ctx, x, *a, **k: None),
+    "a constant": lambda m: setattr(m.layers[2].mixer, "scale", 0.9),
+    "a norm's eps": lambda m: setattr(m.layers[4].norm1, "eps", 0.5),
+    "a weight": lambda m: setattr(m.layers[1].ffn, "w_down", m.layers[1].ffn.w_down * 2),
+    "a weight of other strides": lambda m: setattr(m.layers[2].mixer, "w_o", m.layers[2].mixer.w_o.T),
+    "a bias that was not there": lambda m: setattr(m.layers[2].mixer, "b_o", torch.ones(64)),
+    "another part": lambda m: setattr(m.layers[2], "ffn", _other_ffn(m)),
+    "another layer": lambda m: m.layers.__setitem__(3, _new_layer(m)),
+    "a norm taken from another layer": lambda m: setattr(m.layers[3], "norm1", m.layers[5].norm1),
+}
+
+
+@pytest.mark.parametrize("what", list(CHANGES))
+def test_what_is_changed_after_binding_counts(emu, what):
+    model = _model()
+    before = _steps(model, record=False)
+    CHANGES[what](model)
+    want = _steps(model, record=False)
+    assert not torch.equal(want, before)
+    assert torch.equal(_steps(model), want)
+
+
+# ---- the CUDA backend's own recording ----------------------------------------------------------------------------------
+class Library:
+    """Functions of any name that note their arguments' values and succeed."""
+
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        def fn(*args):
+            self.calls.append((name, [a.value if isinstance(a, ctypes._SimpleCData) else a for a in args]))
+            return 0
+        fn.__name__ = name
+        setattr(self, name, fn)
+        return fn
+
+
+def _native():
+    from hfcpu_b200.kernels.native import NativeBackend
+    b = object.__new__(NativeBackend)
+    lib = Library()
+    b.launches = 0
+    b.__dict__["_lib" if isinstance(vars(NativeBackend).get("lib"), property) else "lib"] = lib
+    return b, lib
+
+
+def _recorded(b, tensors):
+    from hfcpu_b200.kernels.native import _p
+
+    def run():
+        b._check(b.lib.hfb_thing(ctypes.c_int(3), *[_p(t) for t in tensors]), "thing")
+        return "out"
+    return b.record(run, tensors)
+
+
+def test_recording_makes_the_calls_with_other_pointers():
+    b, lib = _native()
+    one = [torch.zeros(512, dtype=torch.uint8), None, torch.zeros(4, 64)]
+    two = [torch.zeros(512, dtype=torch.uint8), None, torch.zeros(4, 64)]
+    out, rec = _recorded(b, one)
+    # (pointers agree in their low bits with the recorded ones, or the layer runs its own code)
+    ok = all((x.data_ptr() ^ y.data_ptr()) & 255 == 0 for x, y in zip(one, two) if x is not None)
+    assert out == "out" and b.launches == 1
+    assert rec.replay(two) == ok
+    if ok:
+        assert lib.calls[1] == ("hfb_thing", [3, two[0].data_ptr(), None, two[2].data_ptr()]) and b.launches == 2
+
+
+def test_recording_refuses_tensors_of_another_form():
+    b, lib = _native()
+    store = torch.zeros(1 << 16)
+    base = -store.data_ptr() % 256 // 4
+
+    def at(offset, *shape, dtype=None):
+        t = store[base + offset:base + offset + 4096][:torch.Size(shape).numel()].view(*shape)
+        return t if dtype is None else t.view(dtype)
+    one = [at(0, 8, 8), at(4096, 64)]
+    _, rec = _recorded(b, one)
+    assert rec.replay([at(8192, 8, 8), at(12288, 64)]) and len(lib.calls) == 2
+    for other in ([at(8192, 8, 8).T, at(12288, 64)],                                    # strides
+                  [at(8192, 4, 16), at(12288, 64)], [at(8192, 8, 8), at(12288, 32)],     # shapes
+                  [at(8192, 8, 8, dtype=torch.int32), at(12288, 64)],                    # type
+                  [at(8192 + 1, 8, 8), at(12288, 64)],                                   # alignment
+                  [None, at(12288, 64)], [at(8192, 8, 8)], [at(8192, 8, 8), at(12288, 64), at(0, 8)]):
+        assert not rec.replay(other)
+    assert len(lib.calls) == 2 and b.launches == 2
