@@ -7,6 +7,7 @@ the host-side logic on a machine without a GPU.)
 """
 from __future__ import annotations
 
+import sys
 from typing import Optional
 
 import torch
@@ -82,10 +83,30 @@ def backend():
     return _backend
 
 
+class Written:
+    """The functions of some classes and modules as they were when this was made, for code that passes them by: what has been put
+    in one's place since (a probe, a wrapper that counts) wants to be called."""
+
+    def __init__(self, *spaces):
+        self._kept = []
+        for s in spaces:
+            own = {n: f for n, f in vars(s).items() if callable(f) or isinstance(f, (property, staticmethod, classmethod))}
+            # (a class may get a function of a name that only its bases had; a module's new names are nobody's)
+            self._kept.append((vars(s), len(vars(s)) if isinstance(s, type) else None, tuple(own), tuple(own.values())))
+        self.names = frozenset(n for _, _, names, _ in self._kept for n in names)
+
+    def holds(self) -> bool:
+        return all((size is None or len(space) == size) and tuple(map(space.get, names)) == functions
+                   for space, size, names, functions in self._kept)
+
+
 def recorder():
     """``record(run, tensors) -> (what run returned, recording)`` of a backend that can make a layer's launches again for layers
-    like it, or None (also while a step is profiled phase by phase)."""
-    return None if profile.enabled else getattr(backend(), "record", None)
+    like it, or None: also while a step is profiled phase by phase, where a function of this module has been replaced, and for a
+    backend whose class has no ``record`` of its own (one that wraps another or derives from it wants to see every call).  The
+    recording is None where none could be made."""
+    b = backend()
+    return b.record if not profile.enabled and "record" in vars(type(b)) and _written.holds() else None
 
 
 def set_backend(b) -> None:
@@ -1020,3 +1041,6 @@ def check_device_errors() -> None:
     word = b.error_word() if hasattr(b, "error_word") else 0
     if word:
         raise DeviceFault(word)
+
+
+_written = Written(sys.modules[__name__])

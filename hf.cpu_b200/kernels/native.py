@@ -12,7 +12,7 @@ from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
 
-from . import build as _build
+from . import Written, build as _build
 
 HFB_ENOTSUP = 2          # status of csrc/hfb200.h: not a case for this kernel, nothing was launched
 
@@ -148,7 +148,10 @@ class NativeBackend:
         return getattr(_tls, "recording", None) or self._lib
 
     def record(self, run, tensors):
-        """``run()`` with its launches written down: (what it returned, the recording)."""
+        """``run()`` with its launches written down: (what it returned, the recording); the recording is None where one of this
+        backend's functions isn't the one written here (what has taken its place would not see the launches made again)."""
+        if not (_written.holds() and _written.names.isdisjoint(vars(self))):
+            return run(), None
         rec, before = Recording(self, tensors), self.launches
         _tls.recording = rec
         try:
@@ -886,3 +889,6 @@ class NativeBackend:
         if w.value and self._counters is not None:
             self._counters.zero_()             # a kernel that gave up may have left tile counts behind
         return w.value
+
+
+_written = Written(NativeBackend)

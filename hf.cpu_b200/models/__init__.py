@@ -138,18 +138,19 @@ class Model:
                 if (e.enter is None and following.enter is None and e.cache_of is None and l.ffn is not None and l.norm2 is not None
                         and not l.post_norms() and l.mixer.state_spec() is None):
                     parts = (l.block, after.block) + self._replay_parts(i)
-                    keys = tuple(p.replay_key() if isinstance(p, Part) else None for p in parts)
+                    keys = tuple(p.replay_key() if isinstance(p, Part) and p.written.names.isdisjoint(vars(p)) else None for p in parts)
                     if all(k is not None for k in keys):
                         key = keys
                         watched += [l, after, *parts]
             self._alike.append(None if key is None else numbers.setdefault(key, len(numbers)))
         self._watched = [(o, o.changes) for o in {id(o): o for o in watched}.values()]      # layers and parts, as they were
         self._layers_then = list(self.layers)
+        self._classes = {type(o) for o in watched if isinstance(o, Part)}
 
     def _alike_now(self) -> Optional[List[Optional[int]]]:
         """``_alike``, None where no entries are.  What has been changed since the weights were bound (an attribute of a part, a
         function put over one of its own, another part in its place) is alike with nothing: its own code runs."""
-        if not self._watched:
+        if not self._watched or not all(c.written.holds() for c in self._classes):
             return None
         if all(o.changes == n for o, n in self._watched) and len(self.layers) == len(self._layers_then) and \
                 all(a is b for a, b in zip(self.layers, self._layers_then)):

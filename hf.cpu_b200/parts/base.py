@@ -15,6 +15,7 @@ from typing import Any, Callable, Dict, List, Optional, Tuple
 
 import torch
 
+from .. import kernels
 from ..config.base import ConfigError, PartSpec
 from ..weights.loader import TensorSpec
 
@@ -89,6 +90,11 @@ class Part:
     # how many times an attribute has been set or taken away: what was found out about a part holds while this stays
     changes = 0
 
+    def __init_subclass__(cls, **more):
+        super().__init_subclass__(**more)
+        cls.written = None
+        cls.written = kernels.Written(*cls.__mro__[:-1])
+
     def __setattr__(self, name, value):
         super().__setattr__(name, value)
         vars(self)["changes"] = self.changes + 1
@@ -100,7 +106,7 @@ class Part:
     def replay_key(self):
         """What two parts have in common whose kernels differ in nothing but :meth:`replay_tensors`, as a hashable value; None for a
         part that launches anything else than this engine's kernels, or reads something of the step on the host.  Asked for once, when
-        the weights are bound: a part that is changed afterwards runs its own code again."""
+        the weights are bound: a part that is changed afterwards, or of whose class a function is replaced, runs its own code again."""
         return None
 
     def replay_tensors(self) -> tuple:

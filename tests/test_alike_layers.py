@@ -129,6 +129,54 @@ def test_what_is_changed_after_binding_counts(emu, what):
     assert torch.equal(_steps(model), want)
 
 
+def test_a_probe_put_over_a_method_sees_every_layer(emu, monkeypatch):
+    from hfcpu_b200 import kernels
+    from hfcpu_b200.parts.attention import OutputProduct, PagedAttention
+    from hfcpu_b200.parts.ffn import SwiGlu
+    model = _model()
+    for owner, name in ((SwiGlu, "_hidden"), (OutputProduct, "forward_then_norm"), (PagedAttention, "forward_then_norm"), (kernels, "linear_glu"),
+                        (kernels, "paged_attention")):
+        seen, inner = [], getattr(owner, name)
+
+        def probe(*args, **kw):
+            seen.append(1)
+            return inner(*args, **kw)
+        with monkeypatch.context() as m:
+            m.setattr(owner, name, probe)
+            _steps(model)
+        assert len(seen) == 3 * 6, (owner, name)
+    before = emu.replayed
+    _steps(model)
+    assert emu.replayed == before + 3 * 3              # and with everything back in its place layers are made again
+
+
+def test_a_backend_around_another_sees_every_call(emu):
+    from hfcpu_b200 import kernels
+
+    class Around:
+        def __init__(self, inner):
+            self.inner, self.calls = inner, 0
+
+        def __getattr__(self, name):
+            return getattr(self.inner, name)
+
+        def paged_attention(self, *args, **kw):
+            self.calls += 1
+            return self.inner.paged_attention(*args, **kw)
+
+    class Derived(RecordingEmu):
+        calls = 0
+
+        def paged_attention(self, *args, **kw):
+            Derived.calls += 1
+            return super().paged_attention(*args, **kw)
+    model = _model()
+    for b in (Around(emu), Derived()):
+        kernels.set_backend(b)
+        _steps(model)
+        assert b.calls == 3 * 6
+
+
 # ---- the CUDA backend's own recording ----------------------------------------------------------------------------------
 class Library:
     """Functions of any name that note their arguments' values and succeed."""
@@ -194,3 +242,16 @@ def test_recording_refuses_tensors_of_another_form():
                   [None, at(12288, 64)], [at(8192, 8, 8)], [at(8192, 8, 8), at(12288, 64), at(0, 8)]):
         assert not rec.replay(other)
     assert len(lib.calls) == 2 and b.launches == 2
+
+
+def test_a_changed_backend_is_not_recorded(monkeypatch):
+    from hfcpu_b200.kernels.native import NativeBackend
+    t = [torch.zeros(8)]
+    b, _ = _native()
+    b.linear = lambda *a: None
+    assert _recorded(b, t) == ("out", None)
+    b, _ = _native()
+    with monkeypatch.context() as m:
+        m.setattr(NativeBackend, "rmsnorm", lambda *a: None)
+        assert _recorded(b, t) == ("out", None)
+    assert _recorded(b, t)[1] is not None
