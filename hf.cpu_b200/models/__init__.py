@@ -124,7 +124,8 @@ class Model:
         return l.norm1, l.mixer, l.norm2, l.ffn, self.layers[self.plan.schedule[i + 1].layer].norm1
 
     def _replay_tensors(self, i: int, cache):
-        return tuple(t for p in self._replay_parts(i) for t in p.replay_tensors()) + (cache.k, cache.v)
+        own = tuple(t for p in self._replay_parts(i) for t in p.replay_tensors())
+        return own if cache is None else own + (cache.k, cache.v)
 
     def _look_for_alike(self) -> None:
         """``_alike``: for each schedule entry a number that entries share whose kernels differ in their tensors only; None for the
@@ -199,7 +200,7 @@ class Model:
             alike = alikes[i] if alikes is not None else None
             if alike is not None:
                 cache = ctx.entry_cache(i)
-                like = alike, None if xn is None else xn.data_ptr(), cache.group
+                like = alike, None if xn is None else xn.data_ptr(), None if cache is None else cache.group
                 if model is not None and model[0] == like and model[1].replay(self._replay_tensors(i, cache)):
                     xn = model[2]
                     continue

@@ -177,6 +177,56 @@ def test_a_backend_around_another_sees_every_call(emu):
         assert b.calls == 3 * 6
 
 
+def _model_of(make_mixer, block=None):
+    """Six layers with mixers (and blocks) made here."""
+    from hfcpu_b200.config import config_from_dict
+    from hfcpu_b200.models import Model
+    from hfcpu_b200.weights import RandomSource
+    model = Model(config_from_dict(CFG), torch.float32, torch.device("cpu"))
+    for i, l in enumerate(model.layers):
+        l.mixer = make_mixer(i)
+        if block is not None:
+            l.block = block()
+    return model.bind(RandomSource(model.tensor_specs(), 3, torch.float32, model.device, std=0.2))
+
+
+def _plain_mixer():
+    from hfcpu_b200 import kernels
+    from hfcpu_b200.parts import Mixer
+    from hfcpu_b200.weights import TensorSpec
+
+    class Straight(Mixer):
+        """x += W norm(x): no cache, no state."""
+        graph_safe = True
+
+        def __init__(self, i):
+            self.name, self.w = f"straight.{i}", None
+
+        def tensor_specs(self):
+            return [TensorSpec(self.name, (64, 64))]
+
+        def bind(self, tensors, run_dtype, device):
+            self.w = tensors[self.name].contiguous()
+
+        def replay_key(self):
+            return ("straight",)
+
+        def replay_tensors(self):
+            return (self.w,)
+
+        def forward(self, ctx, xn, residual, cache, state, write_cache):
+            assert cache is None
+            kernels.linear(xn, self.w, None, residual, accumulate=True)
+    return Straight
+
+
+def test_mixers_without_a_cache(emu):
+    model = _model_of(_plain_mixer())
+    assert model._alike[:5] == [0] * 5
+    want = _steps(model, record=False)
+    assert torch.equal(_steps(model), want) and emu.replayed == 3 * 3
+
+
 # ---- the CUDA backend's own recording ----------------------------------------------------------------------------------
 class Library:
     """Functions of any name that note their arguments' values and succeed."""
