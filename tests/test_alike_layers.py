@@ -227,6 +227,28 @@ def test_mixers_without_a_cache(emu):
     assert torch.equal(_steps(model), want) and emu.replayed == 3 * 3
 
 
+def test_a_block_with_state_of_its_own_is_alike_with_none(emu):
+    from hfcpu_b200.parts import StateSpec
+    from hfcpu_b200.parts.block import PreNormResidual
+
+    class Counting(PreNormResidual):
+        """Adds how many tokens its layer has seen to the stream."""
+
+        def replay_key(self):
+            return ("counting",)
+
+        def state_spec(self):
+            return StateSpec((1,))
+
+        def forward(self, ctx, x, *args, block_state=None, **kw):
+            x.add_(block_state[ctx.seq_slots.long()])
+            block_state[ctx.seq_slots.long()] += x.shape[0]
+            return super().forward(ctx, x, *args, **kw)
+    model = _model_of(_plain_mixer(), Counting)
+    want = _steps(model, record=False)
+    assert torch.equal(_steps(model), want)
+
+
 # ---- the CUDA backend's own recording ----------------------------------------------------------------------------------
 class Library:
     """Functions of any name that note their arguments' values and succeed."""
