@@ -94,6 +94,9 @@ class Written:
             # (a class may get a function of a name that only its bases had; a module's new names are nobody's)
             self._kept.append((vars(s), len(vars(s)) if isinstance(s, type) else None, tuple(own), tuple(own.values())))
         self.names = frozenset(n for _, _, names, _ in self._kept for n in names)
+        self.found = {}                                   # a class's functions by name, its bases' behind its own
+        for _, _, names, functions in reversed(self._kept):
+            self.found.update(zip(names, functions))
 
     def holds(self) -> bool:
         return all((size is None or len(space) == size) and tuple(map(space.get, names)) == functions
@@ -345,7 +348,9 @@ FEW_TOKENS = 8               # most tokens of the products that read the stream 
 def few_tokens(T: int, dtype, norm, *weights, rope=None) -> bool:
     """Whether products of ``T`` tokens with all of these matrices, behind ``norm`` = (weight, eps), are taken from the float32
     stream on: norm, product and what follows it in one kernel each (``rope``: the matrix of :func:`few_rope_kv`; the others go to :func:`few_glu` and :func:`few_linear`)."""
-    takes = getattr(backend(), "few_takes", None)
+    b = backend()
+    # (of the backend's own class: one that wraps another or derives from it may do something with the calls that these stand for)
+    takes = b.few_takes if "few_takes" in vars(type(b)) else None
     return (takes is not None and T <= FEW_TOKENS and dtype == torch.bfloat16 and norm[0].data_ptr() % 16 == 0
             and all(takes(T, w) for w in weights) and (rope is None or takes(T, rope, True)))
 

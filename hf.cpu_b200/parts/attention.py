@@ -298,7 +298,7 @@ class PagedAttention(OutputProduct, Mixer):
 
     def takes_stream(self, ctx, T, norm):
         """Whether :meth:`forward_from_stream` takes a step of ``T`` tokens: the plain rotated layer, few tokens."""
-        return (not self.general and not self.row_norm and self.rotary is not None and self.rotary.n_rot == self.d and self.d in (64, 128)
+        return (self.is_plain(PagedAttention, "forward", "forward_then_norm", "_attend") and not self.general and not self.row_norm and self.rotary is not None and self.rotary.n_rot == self.d and self.d in (64, 128)
                 and kernels.few_tokens(T, ctx.run_dtype, norm, self.w_o, rope=self.w_qkv))
 
     def forward_from_stream(self, ctx, x, norm, cache, write_cache):

@@ -103,6 +103,12 @@ class Part:
         super().__delattr__(name)
         vars(self)["changes"] = self.changes + 1
 
+    def is_plain(self, cls, *names) -> bool:
+        """Whether this is a ``cls`` itself and runs its functions ``names`` as they are written there: asked by code that does their
+        work without calling them."""
+        own, found = vars(self), cls.written.found
+        return type(self) is cls and all(n not in own and getattr(cls, n) is found[n] for n in names)
+
     def replay_key(self):
         """What two parts have in common whose kernels differ in nothing but :meth:`replay_tensors`, as a hashable value; None for a
         part that launches anything else than this engine's kernels, or reads something of the step on the host.  Asked for once, when
@@ -180,6 +186,9 @@ class Mixer(Part):
     # Optional: ``operand_width`` (not None) and ``operand(ctx, xn, cache, state, write_cache, out)``: writes the operand of
     # the mixer's output product (``w_o``, ``b_o``) into ``out`` [T, operand_width], which may be a column slice of a wider
     # array, and leaves the product to the caller.
+    # Optional: ``takes_stream(ctx, T, norm) -> bool`` and ``forward_from_stream(ctx, x, norm, cache, write_cache)``: the whole
+    # sublayer, the norm in front (weight and eps of an RMSNorm) included, for steps of few tokens.  They stand for the other forms
+    # of forward: a class that derives from one that has them and changes what it computes must not say that it takes the stream.
 
 
 class FeedForward(Part):
@@ -188,7 +197,7 @@ class FeedForward(Part):
         raise NotImplementedError
 
     # Optional: ``forward_then_norm(ctx, xn, residual, norm, out) -> bool``, and ``operand_width`` with ``operand(ctx, xn, out)``
-    # (the product being ``w_down``, ``b_down``), as for mixers.
+    # (the product being ``w_down``, ``b_down``), and ``takes_stream`` with ``forward_from_stream(ctx, x, norm)``, as for mixers.
 
 
 class Block(Part):

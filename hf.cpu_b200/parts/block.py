@@ -11,7 +11,7 @@ from .. import kernels
 from ..config.base import UnsupportedError
 from ..weights.loader import TensorSpec
 from .base import Block, StateSpec, register_part
-from .norm import ShiftedNorm
+from .norm import RmsNorm, ShiftedNorm
 
 
 class PreNormResidual(Block):
@@ -50,8 +50,11 @@ class PreNormResidual(Block):
         T = x.shape[0]
         if T > kernels.FEW_TOKENS or not (hasattr(mixer, "takes_stream") and hasattr(ffn, "takes_stream")):
             return False
+        # (the kernels compute the norm themselves: norms that are something else, or more, run their own code)
+        if not all(isinstance(n, RmsNorm) and n.is_plain(RmsNorm, "forward", "fused_args") for n in (norm1, norm2)):
+            return False
         n1, n2 = norm1.fused_args(), norm2.fused_args()
-        if n1 is None or n2 is None or len(n1) != 2 or len(n2) != 2 or not (mixer.takes_stream(ctx, T, n1) and ffn.takes_stream(ctx, T, n2)):
+        if not (mixer.takes_stream(ctx, T, n1) and ffn.takes_stream(ctx, T, n2)):
             return False
         mixer.forward_from_stream(ctx, x, n1, cache, write_cache)
         ffn.forward_from_stream(ctx, x, n2)

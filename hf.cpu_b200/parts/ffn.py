@@ -87,7 +87,7 @@ class SwiGlu(FeedForward):
 
     def takes_stream(self, ctx, T, norm):
         """Whether :meth:`forward_from_stream` takes a step of ``T`` tokens."""
-        return kernels.few_tokens(T, ctx.run_dtype, norm, self.w_gate_up, self.w_down)
+        return self.is_plain(SwiGlu, "forward", "forward_then_norm", "_hidden", "operand") and kernels.few_tokens(T, ctx.run_dtype, norm, self.w_gate_up, self.w_down)
 
     def forward_from_stream(self, ctx, x, norm):
         """``x += feed-forward(norm(x))`` with the norm in the front product's kernel (``norm`` = (weight, eps) of an RMSNorm)."""
