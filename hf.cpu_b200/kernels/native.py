@@ -27,9 +27,6 @@ class KernelError(RuntimeError):
     pass
 
 
-_tls = threading.local()          # .recording: the launches this thread is writing down, if any
-
-
 def _forms(tensors, ptrs):
     """What of tensors the choice of kernels and their arguments may depend on beside the pointers themselves."""
     return [None if t is None else (p & 255, t.shape, t.stride(), t.dtype, t.device) for t, p in zip(tensors, ptrs)]
@@ -41,7 +38,8 @@ class Recording:
     alike layers behind the first make the same calls with their own pointers."""
 
     def __init__(self, backend, tensors):
-        self._backend, self._lib, self._last = backend, backend._lib, None
+        self._backend, self._lib, self._last = backend, backend.lib, None
+        self.thread = threading.get_ident()                # whose launches they are
         self.calls = []
         self.ptrs = [t.data_ptr() if t is not None else 0 for t in tensors]
         self.forms = _forms(tensors, self.ptrs)
@@ -54,7 +52,8 @@ class Recording:
         fn = getattr(self._lib, name)
 
         def call(*args):
-            self._last = fn, args
+            if threading.get_ident() == self.thread:
+                self._last = fn, args
             return fn(*args)
         return call
 
@@ -101,13 +100,14 @@ def _p(t):
 class NativeBackend:
     name = "native"
     lays_out_rows = True         # grouped products of many places take scratch for gathered rows (kernels.moe_wants_rows)
+    _recording, _record_lock = None, threading.Lock()
 
     def __init__(self):
         if not torch.cuda.is_available():
             raise KernelError("no CUDA device is visible: this engine has no CPU path")
         path = _build.build()
         try:
-            self._lib = ctypes.CDLL(path)
+            self.lib = ctypes.CDLL(path)
         except OSError as e:
             raise KernelError(f"the CUDA library {path} could not be loaded: {e}") from None
         self.lib.hfb_last_error.restype = ctypes.c_char_p
@@ -143,21 +143,20 @@ class NativeBackend:
         self.path = path
         self.launches = 0          # kernels launched through this binding (one per successful call)
 
-    @property
-    def lib(self):
-        return getattr(_tls, "recording", None) or self._lib
-
     def record(self, run, tensors):
         """``run()`` with its launches written down: (what it returned, the recording); the recording is None where one of this
-        backend's functions isn't the one written here (what has taken its place would not see the launches made again)."""
-        if not (_written.holds() and _written.names.isdisjoint(vars(self))):
+        backend's functions isn't the one written here (what has taken its place would not see the launches made again), and while
+        another recording is made.  The recording stands in the library's place meanwhile, so that a call costs nothing at other times;
+        other threads' calls go through it unrecorded."""
+        if not (_written.holds() and _written.names.isdisjoint(vars(self))) or not self._record_lock.acquire(blocking=False):
             return run(), None
-        rec, before = Recording(self, tensors), self.launches
-        _tls.recording = rec
+        lib, before = self.lib, self.launches
+        rec = self.lib = self._recording = Recording(self, tensors)
         try:
             out = run()
         finally:
-            _tls.recording = None
+            self.lib, self._recording = lib, None
+            self._record_lock.release()
         rec.count = self.launches - before
         return out, rec
 
@@ -170,8 +169,8 @@ class NativeBackend:
     def _check(self, rc: int, what: str):
         if rc != 0:
             raise KernelError(f"{what}: {self.lib.hfb_last_error().decode()} (status {rc})")
-        rec = getattr(_tls, "recording", None)
-        if rec is not None:
+        rec = self._recording
+        if rec is not None and rec.thread == threading.get_ident():
             rec.add(what)
         self.launches += 1
 

@@ -270,7 +270,7 @@ def _native():
     b = object.__new__(NativeBackend)
     lib = Library()
     b.launches = 0
-    b.__dict__["_lib" if isinstance(vars(NativeBackend).get("lib"), property) else "lib"] = lib
+    b.lib = lib
     return b, lib
 
 
@@ -327,3 +327,37 @@ def test_a_changed_backend_is_not_recorded(monkeypatch):
         m.setattr(NativeBackend, "rmsnorm", lambda *a: None)
         assert _recorded(b, t) == ("out", None)
     assert _recorded(b, t)[1] is not None
+
+
+def test_calls_outside_a_recording_go_straight_to_the_library():
+    """A launch looks the library up two or three times: it is a plain attribute, not asked for through a thread's own storage."""
+    b, lib = _native()
+    assert b.lib is lib and vars(b)["lib"] is lib
+    _recorded(b, [torch.zeros(8)])
+    assert vars(b)["lib"] is lib and b._recording is None
+    with pytest.raises(RuntimeError):
+        b.record(lambda: (_ for _ in ()).throw(RuntimeError("a part's own")), [])
+    assert vars(b)["lib"] is lib and b._recording is None
+    assert _recorded(b, [torch.zeros(8)])[1] is not None
+
+
+def test_another_threads_calls_are_not_in_a_recording():
+    import threading
+    b, lib = _native()
+    t, other = torch.zeros(8), []
+
+    def elsewhere():
+        b._check(b.lib.hfb_elsewhere(ctypes.c_int(1)), "elsewhere")
+        other.append(b.record(lambda: b._check(b.lib.hfb_second(ctypes.c_int(2)), "second"), [t])[1])
+
+    def run():
+        b.lib.hfb_question(ctypes.c_int(0))
+        rc = b.lib.hfb_first(ctypes.c_int(0))
+        th = threading.Thread(target=elsewhere)
+        th.start()
+        th.join()
+        b._check(rc, "first")
+    _, rec = b.record(run, [t])
+    assert other == [None] and [c[0] for c in lib.calls] == ["hfb_question", "hfb_first", "hfb_elsewhere", "hfb_second"]
+    lib.calls.clear()
+    assert rec.replay([t]) and [c[0] for c in lib.calls] == ["hfb_first"]
