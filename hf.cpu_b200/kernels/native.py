@@ -12,7 +12,7 @@ from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
 
-from . import Written, build as _build
+from . import FEW_TOKENS, Written, build as _build
 
 HFB_ENOTSUP = 2          # status of csrc/hfb200.h: not a case for this kernel, nothing was launched
 
@@ -406,7 +406,7 @@ class NativeBackend:
         wherever it takes a product: one / eight tokens, us, few | split product without its tail: 896 x 896 1.9 / 2.6 | 3.3 / 3.5,
         9,728 x 896 5.2 / 5.7 | 6.2 / 6.3, 1,024 x 2,736 2.9 / 3.5 | 3.4 / 3.5, 3,072 x 2,048 3.4 / 3.8 | 4.7 / 4.8; without
         launches that overlap 2.7 / 3.0 | 4.8 / 4.9, 7.0 / 7.4 | 7.9 / 8.1, 4.0 / 4.3 | 5.5 / 5.6, 5.2 / 5.2 | 6.4 / 6.5."""
-        return w.numel() >= 1 << 19 and self.few_takes(a.shape[0], w)
+        return a.shape[0] <= FEW_TOKENS and w.numel() >= 1 << 19 and self.few_takes(a.shape[0], w)
 
     def _partials(self, a, w):
         """Split-K partial sums of a @ w.T in the workspace; returns (workspace, splits)."""

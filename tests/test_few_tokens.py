@@ -128,3 +128,18 @@ def test_a_backend_around_another_sees_the_calls_it_knows(install):
     install(b)
     _steps(_model())
     assert b.calls == 3 * 3
+
+
+def test_products_of_more_tokens_ask_the_library_nothing():
+    """In steps of any size a product is looked at first; the question costs about 1 us of a prompt's host time."""
+    from types import SimpleNamespace
+
+    from hfcpu_b200.kernels.native import NativeBackend
+    asked = []
+    b = object.__new__(NativeBackend)
+    b.gemm, b.lib = "tc", SimpleNamespace(hfb_few_takes=lambda *a: asked.append(a) or 1)
+    w = torch.zeros(1024, 512, dtype=torch.bfloat16)
+    for M, few in ((1, True), (8, True), (9, False), (2000, False)):
+        asked.clear()
+        assert b._few(torch.zeros(M, 512, dtype=torch.bfloat16), w) == few
+        assert len(asked) == few
