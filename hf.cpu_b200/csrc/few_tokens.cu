@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(THREADS, NG <= 8 ? 3 : 2) few_kernel(const Few
     extern __shared__ __align__(128) unsigned char few_sm[];
     float *ss = (float *)few_sm;                               // [MAX_M][WARPS] sums of squares
     unsigned char *sm = few_sm + SS_BYTES;
+    HFB_TRACE_ENTRY(17);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int chunks = (p.K + FEW_CHUNK - 1) / FEW_CHUNK, pieces = chunks * (FEW_CHUNK / 8), stride = few_stride(p.K);
     constexpr int F = NG * 8;

@@ -16,7 +16,8 @@ from . import backend
 
 KERNELS = {1: "gemm", 2: "rope_kv", 3: "attn_decode", 4: "attn_merge", 5: "reduce_norm", 6: "rmsnorm", 7: "embed",
            8: "splitk_reduce", 9: "argmax_chunks", 10: "argmax_final", 11: "reduce_norm_scalar", 12: "attn_fast",
-           13: "attn_tc", 14: "swiglu", 15: "rmsnorm_s", 16: "rope_kv_write"}
+           13: "attn_tc", 14: "swiglu", 15: "rmsnorm_s", 16: "rope_kv_write",
+           17: "few_tokens"}
 MARKS = {0: "entry", 1: "ready", 2: "setup", 3: "issued", 4: "block0_done", 5: "q_in", 6: "tiles_done", 7: "partial_stored",
          8: "last_cta_start", 9: "last_cta_end"}
 CAPACITY = 32768

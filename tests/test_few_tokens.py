@@ -156,3 +156,20 @@ def test_ranges_of_decode_attention():
             assert decode_split_hint(keys) == decode_split_hint(keys, 1) == one, keys
             assert decode_split_hint(keys, 2) == decode_split_hint(keys, 64) == more, keys
     assert decode_split_hint(0) == 1
+
+
+# the sources of the kernels that a step of the first architecture runs
+@pytest.mark.parametrize("name", ["few_tokens", "fused_decode", "gemm_tc", "attention_decode", "attention_fast", "attention_tc", "attention_tc2"])
+def test_every_kernel_of_a_step_is_on_the_timeline(name):
+    """The timeline pairs a kernel's entry with the next wait that returns: one kernel without an entry gives its times to the others."""
+    import os
+    import re
+
+    from hfcpu_b200.kernels import build, timeline
+    with open(os.path.join(build.CSRC, name + ".cu")) as f:
+        source = f.read()
+    bodies = source.split("__global__")[1:]
+    assert bodies
+    for body in bodies:
+        found = re.search(r"HFB_TRACE_ENTRY\((\d+)\)", body)
+        assert found and int(found.group(1)) in timeline.KERNELS, body[:80]
