@@ -267,7 +267,11 @@ static int few_groups(int M, int N, int K, bool pairs)
     return 0;
 }
 
-static bool few_takes(int M, int N, int K, bool pairs) { return M >= 1 && M <= MAX_M && K >= 8 && (K & 7) == 0 && N >= 8 && few_groups(M, N, K, pairs) > 0; }
+// (sizes that no share fits are turned down before the arithmetic on them, which is in 32 bits)
+static bool few_takes(int M, int N, int K, bool pairs)
+{
+    return M >= 1 && M <= MAX_M && K >= 8 && (K & 7) == 0 && K <= FEW_SMEM_MAX && N >= 8 && N <= (1 << 30) && few_groups(M, N, K, pairs) > 0;
+}
 
 static int few_launch(const FewParams &p, cudaStream_t st)
 {

@@ -173,3 +173,18 @@ def test_every_kernel_of_a_step_is_on_the_timeline(name):
     for body in bodies:
         found = re.search(r"HFB_TRACE_ENTRY\((\d+)\)", body)
         assert found and int(found.group(1)) in timeline.KERNELS, body[:80]
+
+
+def test_sizes_beyond_32_bits_of_arithmetic_are_refused():
+    """An inner size just below 2^31 wrapped to a small one when its row in shared memory was counted: the product of it was taken,
+    and would have been sums of nothing."""
+    import ctypes
+
+    from hfcpu_b200.kernels import build
+    lib = ctypes.CDLL(build.build())
+    assert lib.hfb_few_takes(1, 8, 8, 0) == 1
+    for N, K in ((8, 2 ** 31 - 8), (8, 2 ** 31 - 32), (8, 2 ** 30), (2 ** 31 - 1, 8), (2 ** 31 - 8, 2 ** 31 - 8), (8, 1 << 17)):
+        for rope in (0, 1):
+            assert lib.hfb_few_takes(1, N, K, rope) == 0, (N, K)
+    for bad in ((0, 8, 8), (9, 8, 8), (1, 7, 8), (1, 8, 4), (1, 8, 12), (-1, 8, 8), (1, -8, 8), (1, 8, -8)):
+        assert lib.hfb_few_takes(*bad, 0) == 0, bad
