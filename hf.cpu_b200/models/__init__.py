@@ -139,7 +139,7 @@ class Model:
                 if (e.enter is None and following.enter is None and e.cache_of is None and l.ffn is not None and l.norm2 is not None
                         and not l.post_norms() and l.mixer.state_spec() is None and l.block.state_spec() is None):
                     parts = (l.block, after.block) + self._replay_parts(i)
-                    keys = tuple(p.replay_key() if isinstance(p, Part) and p.written.names.isdisjoint(vars(p)) else None for p in parts)
+                    keys = tuple(p.replay_key() if isinstance(p, Part) and p.counts_changes and p.written.names.isdisjoint(vars(p)) else None for p in parts)
                     if all(k is not None for k in keys):
                         key = keys
                         watched += [l, after, *parts]

@@ -249,6 +249,28 @@ def test_a_block_with_state_of_its_own_is_alike_with_none(emu):
     assert torch.equal(_steps(model), want)
 
 
+def test_only_parts_that_may_be_alike_count_their_changes(emu):
+    """Counting costs every attribute of every part that is made; a class that sets attributes its own way is alike with none."""
+    from hfcpu_b200.parts.latent_attention import LatentAttention
+    from hfcpu_b200.parts.norm import DynamicTanh
+    for cls in (LatentAttention, DynamicTanh):
+        assert cls.__setattr__ is object.__setattr__ and not cls.counts_changes
+    Plain = _plain_mixer()
+    part = Plain(0)
+    before = part.changes
+    part.w = 1
+    del part.w
+    assert Plain.counts_changes and part.changes == before + 2
+
+    class Own(Plain):
+        def __setattr__(self, name, value):
+            super().__setattr__(name, value)
+    assert not Own.counts_changes
+    model = _model_of(Own)
+    assert model._alike == [None] * 6
+    assert torch.equal(_steps(model), _steps(model, record=False)) and emu.replayed == 0
+
+
 # ---- the CUDA backend's own recording ----------------------------------------------------------------------------------
 class Library:
     """Functions of any name that note their arguments' values and succeed."""
