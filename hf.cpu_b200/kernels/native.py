@@ -217,7 +217,7 @@ class NativeBackend:
         if (self.gemm == "tc" and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 8 == 0
                 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
                 and (bias is None or bias.data_ptr() % 16 == 0)):
-            if self._few(a, w):
+            if M <= FEW_TOKENS and self._few(a, w):
                 self.few_linear(a, None, w, bias, out, accumulate)
                 return
             need = self.lib.hfb_linear_tc_workspace(c_int(M), c_int(N), c_int(K))
@@ -412,7 +412,7 @@ class NativeBackend:
         M, K = a.shape
         N = w.shape[0]
         ws = self._workspace(a.device)
-        if self._few(a, w):                                     # one plane, the finished sums
+        if M <= FEW_TOKENS and self._few(a, w):                                     # one plane, the finished sums
             self.few_linear(a, None, w, None, ws[:4 * M * N].view(torch.float32), False)
             return ws, 1
         need = self.lib.hfb_linear_tc_partials_workspace(c_int(M), c_int(N), c_int(K))
@@ -429,7 +429,7 @@ class NativeBackend:
         M, K = a.shape
         N = w.shape[0]
         if self._tc_ok(a, w, out):
-            if self._few(a, w):
+            if M <= FEW_TOKENS and self._few(a, w):
                 self.few_glu(a, None, w, None, out, 0, None)
                 return
             self._check(self.lib.hfb_linear_tc_swiglu(_p(a), _p(w), _p(out), c_int(_dt(out)), c_int(M), c_int(N), c_int(K),
@@ -645,10 +645,10 @@ class NativeBackend:
         consts = tuple(c_float(x) for x in (clamp or (0.0, 0.0, 0.0)))
         ldo = c_int64(out.stride(0))
         if self._tc_ok(a, w, out):
-            if self._few(a, w):
+            M, K = a.shape
+            if M <= FEW_TOKENS and self._few(a, w):
                 self.few_glu(a, None, w, bias, out, act, clamp)
                 return
-            M, K = a.shape
             self._check(self.lib.hfb_linear_tc_glu(_p(a), _p(w), _p(bias), b_dt, _p(out), c_int(_dt(out)), ldo, c_int(M), c_int(w.shape[0]),
                                                    c_int(K), c_int(act), *consts, self._stream()), "linear_tc_glu")
             return
@@ -660,10 +660,10 @@ class NativeBackend:
     def linear_act(self, a, w, out, act):
         self._on_gpu(a, w, out)
         if self._tc_ok(a, w, out) and 0 < act < 4:
-            if self._few(a, w):
+            M, K = a.shape
+            if M <= FEW_TOKENS and self._few(a, w):
                 self.few_linear(a, None, w, None, out, False, act)
                 return
-            M, K = a.shape
             self._check(self.lib.hfb_linear_tc_act(_p(a), _p(w), _p(out), c_int(_dt(out)), c_int(M), c_int(w.shape[0]), c_int(K),
                                                    c_int(act), self._stream()), "linear_tc_act")
             return

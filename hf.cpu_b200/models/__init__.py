@@ -191,7 +191,7 @@ class Model:
         for tr in self.transitions.values():
             tr.begin(ctx, x)
         xn = None                                # norm1 of the coming block, when the previous block computed it
-        record = kernels.recorder()
+        record = kernels.recorder() if self._watched else None
         alikes = self._alike_now() if record is not None else None
         model = None                             # ((number, input, cache group), launches, output) of a layer that was written down
         for i, e in enumerate(schedule):
