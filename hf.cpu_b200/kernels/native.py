@@ -83,6 +83,7 @@ class Recording:
 
 
 F32, BF16 = 0, 1
+_ZERO = c_float(0.0)
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -128,6 +129,7 @@ class NativeBackend:
         self._argmax_ws = None
         # decode attention: the CTA that stores a tile's last split merges the splits (False: a second kernel does)
         self.merge_in_kernel = True
+        self._few_sizes = {}                      # (tokens, features, inner size, rope) -> whether the kernel of few tokens has it
         self.rope_in_epilogue = os.environ.get("HFB_ROPE_EPILOGUE", "1") != "0"     # prompts: q|k|v product rotates and writes the cache
         self._counters = None
         self.branches = os.environ.get("HFB_BRANCHES", "1") != "0"        # independent work of a captured step as branches of the graph
@@ -218,7 +220,7 @@ class NativeBackend:
                 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
                 and (bias is None or bias.data_ptr() % 16 == 0)):
             if M <= FEW_TOKENS and self._few(a, w):
-                self.few_linear(a, None, w, bias, out, accumulate)
+                self._few_linear(a, w, bias, _p(out), _dt(out), accumulate)
                 return
             need = self.lib.hfb_linear_tc_workspace(c_int(M), c_int(N), c_int(K))
             if need:
@@ -405,7 +407,7 @@ class NativeBackend:
         wherever it takes a product: one / eight tokens, us, few | split product without its tail: 896 x 896 1.9 / 2.6 | 3.3 / 3.5,
         9,728 x 896 5.2 / 5.7 | 6.2 / 6.3, 1,024 x 2,736 2.9 / 3.5 | 3.4 / 3.5, 3,072 x 2,048 3.4 / 3.8 | 4.7 / 4.8; without
         launches that overlap 2.7 / 3.0 | 4.8 / 4.9, 7.0 / 7.4 | 7.9 / 8.1, 4.0 / 4.3 | 5.5 / 5.6, 5.2 / 5.2 | 6.4 / 6.5."""
-        return a.shape[0] <= FEW_TOKENS and w.numel() >= 1 << 19 and self.few_takes(a.shape[0], w)
+        return a.shape[0] <= FEW_TOKENS and w.numel() >= 1 << 19 and self._few_has(a.shape[0], *w.shape, 0)
 
     def _partials(self, a, w):
         """Split-K partial sums of a @ w.T in the workspace; returns (workspace, splits)."""
@@ -413,7 +415,7 @@ class NativeBackend:
         N = w.shape[0]
         ws = self._workspace(a.device)
         if M <= FEW_TOKENS and self._few(a, w):                                     # one plane, the finished sums
-            self.few_linear(a, None, w, None, ws[:4 * M * N].view(torch.float32), False)
+            self._few_linear(a, w, None, _p(ws), F32, False)
             return ws, 1
         need = self.lib.hfb_linear_tc_partials_workspace(c_int(M), c_int(N), c_int(K))
         if need == 0 or need > ws.numel():                      # 0: above 128 rows, and not a product that is split
@@ -430,7 +432,7 @@ class NativeBackend:
         N = w.shape[0]
         if self._tc_ok(a, w, out):
             if M <= FEW_TOKENS and self._few(a, w):
-                self.few_glu(a, None, w, None, out, 0, None)
+                self._few_glu(a, w, None, out, 0, None)
                 return
             self._check(self.lib.hfb_linear_tc_swiglu(_p(a), _p(w), _p(out), c_int(_dt(out)), c_int(M), c_int(N), c_int(K),
                                                       self._stream()), "linear_tc_swiglu")
@@ -499,7 +501,28 @@ class NativeBackend:
     # ---- a few tokens: norm, product and what follows it in one kernel -------------------------------------
     def few_takes(self, M, w, rope=False):
         return (self.gemm == "tc" and w.dtype == torch.bfloat16 and w.data_ptr() % 16 == 0
-                and bool(self.lib.hfb_few_takes(c_int(M), c_int(w.shape[0]), c_int(w.shape[1]), c_int(1 if rope else 0))))
+                and self._few_has(M, w.shape[0], w.shape[1], 1 if rope else 0))
+
+    def _few_has(self, *sizes):
+        """The library's answer for (tokens, features, inner size, rope), which depends on nothing else; kept, since asking takes 1 us."""
+        has = self._few_sizes.get(sizes)
+        if has is None:
+            if len(self._few_sizes) >= 4096:
+                self._few_sizes.clear()
+            has = self._few_sizes[sizes] = bool(self.lib.hfb_few_takes(*map(c_int, sizes)))
+        return has
+
+    # (two forms for products whose operands have been looked at; plain numbers go to the library as ints)
+    def _few_linear(self, a, w, bias, out_ptr, out_dt, accumulate, act=0):
+        N, K = w.shape
+        self._check(self.lib.hfb_few_linear(_p(a), None, 0, _ZERO, _p(w), _p(bias), _dt(bias) if bias is not None else 0, out_ptr, out_dt,
+                                            1 if accumulate else 0, act, a.shape[0], N, K, self._stream()), "few_linear")
+
+    def _few_glu(self, a, w, bias, out, act, clamp):
+        N, K = w.shape
+        limit, alpha, offset = map(c_float, clamp) if clamp else (_ZERO, _ZERO, _ZERO)
+        self._check(self.lib.hfb_few_glu(_p(a), None, 0, _ZERO, _p(w), _p(bias), _dt(bias) if bias is not None else 0, _p(out), _dt(out),
+                                         c_int64(out.stride(0)), a.shape[0], N, K, act, limit, alpha, offset, self._stream()), "few_glu")
 
     def _few_in(self, a, norm, w):
         nw, eps = norm or (None, 0.0)
@@ -641,14 +664,15 @@ class NativeBackend:
     def linear_glu(self, a, w, gu_buf, out, act, bias=None, clamp=None):
         self._on_gpu(a, w, bias)
         self._rows_on_gpu(out)
+        M, K = a.shape
+        tc = self._tc_ok(a, w, out)
+        if tc and M <= FEW_TOKENS and self._few(a, w):
+            self._few_glu(a, w, bias, out, act, clamp)
+            return
         b_dt = c_int(_dt(bias) if bias is not None else 0)
         consts = tuple(c_float(x) for x in (clamp or (0.0, 0.0, 0.0)))
         ldo = c_int64(out.stride(0))
-        if self._tc_ok(a, w, out):
-            M, K = a.shape
-            if M <= FEW_TOKENS and self._few(a, w):
-                self.few_glu(a, None, w, bias, out, act, clamp)
-                return
+        if tc:
             self._check(self.lib.hfb_linear_tc_glu(_p(a), _p(w), _p(bias), b_dt, _p(out), c_int(_dt(out)), ldo, c_int(M), c_int(w.shape[0]),
                                                    c_int(K), c_int(act), *consts, self._stream()), "linear_tc_glu")
             return
@@ -662,7 +686,7 @@ class NativeBackend:
         if self._tc_ok(a, w, out) and 0 < act < 4:
             M, K = a.shape
             if M <= FEW_TOKENS and self._few(a, w):
-                self.few_linear(a, None, w, None, out, False, act)
+                self._few_linear(a, w, None, _p(out), _dt(out), False, act)
                 return
             self._check(self.lib.hfb_linear_tc_act(_p(a), _p(w), _p(out), c_int(_dt(out)), c_int(M), c_int(w.shape[0]), c_int(K),
                                                    c_int(act), self._stream()), "linear_tc_act")

@@ -137,12 +137,18 @@ def test_products_of_more_tokens_ask_the_library_nothing():
     from hfcpu_b200.kernels.native import NativeBackend
     asked = []
     b = object.__new__(NativeBackend)
-    b.gemm, b.lib = "tc", SimpleNamespace(hfb_few_takes=lambda *a: asked.append(a) or 1)
+    b.gemm, b._few_sizes, b.lib = "tc", {}, SimpleNamespace(hfb_few_takes=lambda *a: asked.append(a) or 1)
     w = torch.zeros(1024, 512, dtype=torch.bfloat16)
     for M, few in ((1, True), (8, True), (9, False), (2000, False)):
         asked.clear()
         assert b._few(torch.zeros(M, 512, dtype=torch.bfloat16), w) == few
         assert len(asked) == few
+    asked.clear()
+    assert b._few(torch.zeros(1, 512, dtype=torch.bfloat16), w) and not asked                  # nor a second time about the same sizes
+    for M in range(1, 9):
+        for n in range(1000):
+            b._few_has(M, n, 8, 0)
+    assert len(b._few_sizes) <= 4096                                                           # kept for so many
 
 
 def test_ranges_of_decode_attention():
