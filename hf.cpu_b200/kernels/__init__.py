@@ -92,15 +92,23 @@ class Written:
         for s in spaces:
             own = {n: f for n, f in vars(s).items() if callable(f) or isinstance(f, (property, staticmethod, classmethod))}
             # (a class may get a function of a name that only its bases had; a module's new names are nobody's)
-            self._kept.append((vars(s), len(vars(s)) if isinstance(s, type) else None, tuple(own), tuple(own.values())))
-        self.names = frozenset(n for _, _, names, _ in self._kept for n in names)
+            self._kept.append((s, len(vars(s)) if isinstance(s, type) else None, tuple(own), tuple(own.values()), vars(s)))
+        self.names = frozenset(n for k in self._kept for n in k[2])
         self.found = {}                                   # a class's functions by name, its bases' behind its own
-        for _, _, names, functions in reversed(self._kept):
+        for _, _, names, functions, _ in reversed(self._kept):
             self.found.update(zip(names, functions))
+
+    @classmethod
+    def together(cls, several):
+        """Several as one that only :meth:`holds`."""
+        one = cls()
+        for w in several:
+            one._kept += [k for k in w._kept if k not in one._kept]
+        return one
 
     def holds(self) -> bool:
         return all((size is None or len(space) == size) and tuple(map(space.get, names)) == functions
-                   for space, size, names, functions in self._kept)
+                   for _, size, names, functions, space in self._kept)
 
 
 def recorder():

@@ -27,9 +27,9 @@ class KernelError(RuntimeError):
     pass
 
 
-def _forms(tensors, ptrs):
-    """What of tensors the choice of kernels and their arguments may depend on beside the pointers themselves."""
-    return [None if t is None else (p & 255, t.shape, t.stride(), t.dtype, t.device) for t, p in zip(tensors, ptrs)]
+def _forms(tensors):
+    """What of tensors the choice of kernels and their arguments may depend on beside their addresses."""
+    return [None if t is None else (t.shape, t.dtype, t.is_cuda, t.is_contiguous(), t.data_ptr() & 255) for t in tensors]
 
 
 class Recording:
@@ -40,12 +40,12 @@ class Recording:
     def __init__(self, backend, tensors):
         self._backend, self._lib, self._last = backend, backend.lib, None
         self.thread = threading.get_ident()                # whose launches they are
-        self.calls = []
-        self.ptrs = [t.data_ptr() if t is not None else 0 for t in tensors]
-        self.forms = _forms(tensors, self.ptrs)
-        known = [p for p in self.ptrs if p]
-        self.index = {p: k for k, p in enumerate(self.ptrs) if p}
-        self.sound = len(known) == len(self.index)         # (a tensor in two places could not be told apart in another layer)
+        self.calls = []                                    # (function, arguments, what it is)
+        self.forms = _forms(tensors)
+        self.places = [c_void_p(t.data_ptr()) if t is not None else None for t in tensors]   # the arguments that stand for the tensors
+        self.index = {p.value: p for p in self.places if p is not None}
+        # (a tensor in two places could not be told apart in another layer; rows with gaps are no kernel's operands as they are)
+        self.sound = len(self.index) == sum(p is not None for p in self.places) and all(f is None or f[3] for f in self.forms)
         self.count = 0                                     # kernels the calls launch
 
     def __getattr__(self, name):
@@ -60,21 +60,17 @@ class Recording:
     def add(self, what):
         """Keeps the call that was made last: its result has been checked, so it was a launch and no question."""
         fn, args = self._last
-        own = [(at, self.index[a.value]) for at, a in enumerate(args) if isinstance(a, c_void_p) and a.value in self.index]
-        self.calls.append((fn, args, own, what))
+        self.calls.append((fn, [self.index.get(a.value, a) if isinstance(a, c_void_p) else a for a in args], what))
 
     def replay(self, tensors) -> bool:
         """Makes the calls with these tensors in the places of the recorded layer's; False, with nothing launched, where one is
-        missing that was there, aligned otherwise, or of another shape, stride, type or device."""
-        ptrs = [t.data_ptr() if t is not None else 0 for t in tensors]
-        if not self.sound or self.forms != _forms(tensors, ptrs):
+        missing that was there, aligned otherwise, of another shape or type, on another kind of device or not contiguous."""
+        if not self.sound or self.forms != _forms(tensors):
             return False
-        ptrs = [c_void_p(p) for p in ptrs]
-        for fn, args, own, what in self.calls:
-            if own:
-                args = list(args)
-                for at, k in own:
-                    args[at] = ptrs[k]
+        for place, t in zip(self.places, tensors):
+            if place is not None:
+                place.value = t.data_ptr()
+        for fn, args, what in self.calls:
             rc = fn(*args)
             if rc != 0:
                 raise KernelError(f"{what}: {self._lib.hfb_last_error().decode()} (status {rc})")

@@ -6,12 +6,14 @@ entries in order, then the final norm and the head on the rows whose logits are 
 """
 from __future__ import annotations
 
+import operator
 import os
 from dataclasses import dataclass
 from typing import Dict, List, Optional
 
 import torch
 
+from .. import kernels
 from ..config import ModelConfig, load_config
 from ..config.base import ModelPlan
 from ..parts import Part, make_part
@@ -144,19 +146,20 @@ class Model:
                         key = keys
                         watched += [l, after, *parts]
             self._alike.append(None if key is None else numbers.setdefault(key, len(numbers)))
-        self._watched = [(o, o.changes) for o in {id(o): o for o in watched}.values()]      # layers and parts, as they were
-        self._layers_then = list(self.layers)
-        self._classes = {type(o) for o in watched if isinstance(o, Part)}
+        # layers and parts as they were, and the functions of their classes
+        self._watched = list({id(o): o for o in watched}.values())
+        self._changes_then, self._layers_then = [o.changes for o in self._watched], list(self.layers)
+        self._written = kernels.Written.together(c.written for c in {type(o): None for o in self._watched if isinstance(o, Part)})
 
     def _alike_now(self) -> Optional[List[Optional[int]]]:
         """``_alike``, None where no entries are.  What has been changed since the weights were bound (an attribute of a part, a
         function put over one of its own, another part in its place) is alike with nothing: its own code runs."""
-        if not self._watched or not all(c.written.holds() for c in self._classes):
+        if not self._watched or not self._written.holds():
             return None
-        if all(o.changes == n for o, n in self._watched) and len(self.layers) == len(self._layers_then) and \
-                all(a is b for a, b in zip(self.layers, self._layers_then)):
+        if [o.changes for o in self._watched] == self._changes_then and len(self.layers) == len(self._layers_then) and \
+                all(map(operator.is_, self.layers, self._layers_then)):
             return self._alike
-        same = {id(o) for o, n in self._watched if o.changes == n}
+        same = {id(o) for o, n in zip(self._watched, self._changes_then) if o.changes == n}
         out = []
         for i, number in enumerate(self._alike):
             if number is not None:
@@ -177,7 +180,6 @@ class Model:
 
     # ---- forward ------------------------------------------------------------------------
     def forward(self, ctx) -> Optional[torch.Tensor]:
-        from .. import kernels
         T = ctx.token_ids.shape[0]
         S = self.plan.streams
         x = ctx.buf("residual", (T, self.plan.hidden_size), torch.float32)
