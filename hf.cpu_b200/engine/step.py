@@ -340,7 +340,7 @@ class Engine:
         ctx.h_cu_tokens, ctx.h_kv_lens, ctx.h_seq_slots = cu, kv_lens, seq_slots
         ctx.max_q_len = max_q
         ctx.max_kv_len = max(kv_lens)
-        ctx.decode_split_hint = kernels.decode_split_hint(ctx.max_kv_len, S)
+        ctx.decode_split_hint = kernels.decode_split_hint(ctx.max_kv_len)
         return ctx
 
     def _replay(self, ctx: StepContext) -> torch.Tensor:

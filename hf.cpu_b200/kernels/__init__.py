@@ -125,22 +125,18 @@ def set_backend(b) -> None:
     _backend = b
 
 
-def decode_split_hint(max_kv_len: int, requests: int = 1) -> int:
-    """Into how many ranges decode attention may cut a request's keys, with ``max_kv_len`` keys the longest of ``requests``: a power
-    of two, so that few graphs exist.
+def decode_split_hint(max_kv_len: int) -> int:
+    """Into how many ranges decode attention may cut a request's keys, with ``max_kv_len`` keys the longest: a power of two, so that
+    few graphs exist.
 
     A CTA walks its range in tiles of 64 keys, and the last one merges the ranges, a trip to L2 and back that costs about as much as
-    a few tiles.  Measured: attention and the o product behind it, us a layer, keys and weights out of L2; one range, and 2, 4, 8, 16.
-    Contexts of up to six tiles stay whole: 0.5B sizes, one request, six tiles 8.2, 9.2, 8.9, 8.6, 8.6; 7B sizes, eight requests 18.1,
-    19.0, 18.5, 19.4, 19.4.  Up to 31 tiles one request is cut into one to two tiles a range (7B sizes, 9 tiles 18.7 in four ranges, 17.9 in
-    eight; 28 tiles 21.2 in eight, 18.5 in sixteen).  More requests fill the SMs sooner, and a range is 1.7 to 3.4 tiles: 16 heads of
-    128 over 4, eight requests, 8 tiles 11.3 in four ranges, 12.0 in eight; 12 tiles 12.0, 12.7; 14 tiles 13.6, 13.1; 0.5B sizes, six
-    requests, 16 tiles 9.8 in eight, 10.4 in sixteen; 28 tiles 11.1, 10.5.  From 32 tiles on two to four tiles a range, more beyond
-    8,192 keys (64 ranges at most)."""
+    six tiles.  Short contexts stay whole (0.5B sizes, one token behind 208 / 320 keys, seven steps: 4.72 -> 4.47, 4.79 -> 4.62 ms;
+    512 keys whole 4.93, in eight ranges 4.79); up to 2,048 keys a range is a tile (1,536 keys: eight ranges 5.15, sixteen 4.89 ms; 7B
+    sizes 20.87 -> 20.40); beyond, two tiles."""
     tiles = max(1, (max_kv_len + 63) // 64)
     if tiles <= 6:
         return 1
-    ranges = tiles // 2 if tiles >= 32 else tiles if requests == 1 else tiles * 3 // 5
+    ranges = tiles if tiles < 32 else tiles // 2
     return 1 << (min(ranges, 64).bit_length() - 1)
 
 

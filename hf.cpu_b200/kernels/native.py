@@ -12,7 +12,7 @@ from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
 
-from . import FEW_TOKENS, Written, build as _build, decode_split_hint
+from . import FEW_TOKENS, Written, build as _build
 
 HFB_ENOTSUP = 2          # status of csrc/hfb200.h: not a case for this kernel, nothing was launched
 
@@ -331,7 +331,8 @@ class NativeBackend:
                     groups = G * next(s for s in range(1, H // G + 1) if H // G <= 16 * s and (H // G) % s == 0)
                 if decode:
                     # about `decode_ctas_per_sm` CTAs per SM in all; with one per SM the deep pipeline fits
-                    hint = getattr(ctx, "decode_split_hint", None) or decode_split_hint(ctx.max_kv_len, T)
+                    from . import decode_split_hint
+                    hint = getattr(ctx, "decode_split_hint", None) or decode_split_hint(ctx.max_kv_len)
                     splits = max(1, min(self.decode_ctas_per_sm * self.sm_count // max(1, n_tiles * groups), hint))
                     stages = self.decode_stages
                 else:
