@@ -130,9 +130,13 @@ def decode_split_hint(max_kv_len: int) -> int:
     few graphs exist.
 
     A CTA walks its range in tiles of 64 keys, and the last one merges the ranges, a trip to L2 and back that costs about as much as
-    six tiles.  Short contexts stay whole (0.5B sizes, one token behind 208 / 320 keys, seven steps: 4.72 -> 4.47, 4.79 -> 4.62 ms;
-    512 keys whole 4.93, in eight ranges 4.79); up to 2,048 keys a range is a tile (1,536 keys: eight ranges 5.15, sixteen 4.89 ms; 7B
-    sizes 20.87 -> 20.40); beyond, two tiles."""
+    a few tiles.  Contexts of up to six tiles stay whole; up to 31 tiles a range is one to two tiles, from 32 on two to four, and more
+    beyond 8,192 keys (64 ranges at most).  Whole steps, us, in 1, 2, 4, 8, 16 ranges: 0.5B sizes, one request, six tiles 588, 609, 603,
+    597, 594; 16 tiles 701, 680, 639, 605, 598; 28 tiles 855, 762, 684, 648, 610; eight requests, 12 tiles 823, 820, 762, 753, 747.  Width
+    2,048, eight requests, 12 tiles 543, 543, 525, 517, 514.  Twelve layers of the 7B sizes, one request, 28 tiles 1,509, 1,457, 1,393,
+    1,371, 1,334.  Where the rule is not the best: four to twelve requests of the 7B sizes (seven heads of 128 share a key, the most
+    to merge) at 8, 12, 16 and 24 tiles, 0.3 to 0.9 % of a step (eight requests, 8 tiles 1,392 in four ranges, 1,403 in eight), and 32
+    requests, which fill the SMs whole up to nine tiles, 2 % (7B sizes, 8 tiles 1,514 whole, 1,544)."""
     tiles = max(1, (max_kv_len + 63) // 64)
     if tiles <= 6:
         return 1

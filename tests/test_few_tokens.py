@@ -151,6 +151,15 @@ def test_products_of_more_tokens_ask_the_library_nothing():
     assert len(b._few_sizes) <= 4096                                                           # kept for so many
 
 
+def test_ranges_of_decode_attention():
+    """At the edges of the rule, in tiles of 64 keys."""
+    from hfcpu_b200.kernels import decode_split_hint
+    edges = {1: 1, 6: 1, 7: 4, 8: 8, 15: 8, 16: 16, 31: 16, 32: 16, 63: 16, 64: 32, 127: 32, 128: 64, 4096: 64}
+    for tiles, ranges in edges.items():
+        assert decode_split_hint(tiles * 64 - 63) == decode_split_hint(tiles * 64) == ranges, tiles
+    assert decode_split_hint(0) == 1
+
+
 # the sources of the kernels that a step of the first architecture runs
 @pytest.mark.parametrize("name", ["few_tokens", "fused_decode", "gemm_tc", "attention_decode", "attention_fast", "attention_tc", "attention_tc2"])
 def test_every_kernel_of_a_step_is_on_the_timeline(name):
