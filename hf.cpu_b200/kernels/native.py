@@ -400,10 +400,12 @@ class NativeBackend:
         return self._ws
 
     def _few(self, a, w):
-        """Whether the kernel of few tokens has this product (of operands :meth:`_tc_ok` has looked at).  It is the faster one
-        wherever it takes a product: one / eight tokens, us, few | split product without its tail: 896 x 896 1.9 / 2.6 | 3.3 / 3.5,
-        9,728 x 896 5.2 / 5.7 | 6.2 / 6.3, 1,024 x 2,736 2.9 / 3.5 | 3.4 / 3.5, 3,072 x 2,048 3.4 / 3.8 | 4.7 / 4.8; without
-        launches that overlap 2.7 / 3.0 | 4.8 / 4.9, 7.0 / 7.4 | 7.9 / 8.1, 4.0 / 4.3 | 5.5 / 5.6, 5.2 / 5.2 | 6.4 / 6.5."""
+        """Whether the kernel of few tokens has this product (of operands :meth:`_tc_ok` has looked at).  Where it takes one it was the
+        faster at all of 33 sizes from 128 x 1,024 to 9,728 x 896 and 8,192 x 1,024, with one to eight tokens, weights out of L2, launches
+        overlapping or not.  Of the split product's time: added to a stream 0.38 (896 x 896, one token: 2.3 | 6.1 us) to 0.91 (9,728 x
+        896: 6.0 | 6.6), with a norm's tail behind it 0.70 to 0.99 (2,048 x 4,096, six tokens: 7.7 | 7.8), as a gated pair 0.19 to 0.90.
+        The line at half a million weights is none of speed (128 x 1,024 with its tail, eight tokens: 4.0 | 5.0): below it are
+        mostly the routers' and the low ranks' products, whose sums stay in the order they were in."""
         return a.shape[0] <= FEW_TOKENS and w.numel() >= 1 << 19 and self._few_has(a.shape[0], *w.shape, 0)
 
     def _partials(self, a, w):
