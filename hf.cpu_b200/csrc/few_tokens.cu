@@ -11,7 +11,7 @@
 // The kernel behind is released when the wait returns: released at entry, its copies and those of the one behind it came before this
 // one's (eight steps of one token, 0.5B sizes: 5.07 against 4.63 ms).
 // Measured, a layer of the 0.5B sizes in a step of one token: 30 us with split products and their tails, 21 now; 896 x 896 and
-// 9,728 x 896, one token, where launches do not overlap: 2.7 and 7.0 us, 4.8 and 7.9 the split products without their tails.
+// 9,728 x 896, one token, added to the stream, weights out of L2, launches overlapping: 2.3 and 6.0 us, 6.1 and 6.6 the split products.
 // Every block runs at once, one an SM: the rule (few_groups) takes matrices of which an SM holds its share in shared memory.
 #include "common.cuh"
 
