@@ -126,8 +126,9 @@ class Model:
         return l.norm1, l.mixer, l.norm2, l.ffn, self.layers[self.plan.schedule[i + 1].layer].norm1
 
     def _replay_tensors(self, i: int, cache):
-        own = tuple(t for p in self._replay_parts(i) for t in p.replay_tensors())
-        return own if cache is None else own + (cache.k, cache.v)
+        a, b, c, d, e = self._replay_parts(i)
+        own = (*a.replay_tensors(), *b.replay_tensors(), *c.replay_tensors(), *d.replay_tensors(), *e.replay_tensors())
+        return own if cache is None else (*own, cache.k, cache.v)
 
     def _look_for_alike(self) -> None:
         """``_alike``: for each schedule entry a number that entries share whose kernels differ in their tensors only; None for the
