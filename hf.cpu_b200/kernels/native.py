@@ -57,8 +57,11 @@ class Recording:
             return fn(*args)
         return call
 
-    def add(self, what):
-        """Keeps the call that was made last: its result has been checked, so it was a launch and no question."""
+    def check(self, rc, what):
+        """The backend's ``_check``, and keeps the call that was made last: its result is checked, so it was a launch and no question."""
+        NativeBackend._check(self._backend, rc, what)
+        if threading.get_ident() != self.thread:
+            return
         fn, args = self._last
         # (plain ints and None are what the call converts fastest: 0.4 us of a launch)
         self.calls.append((fn, [(self.index.get(a.value, a) if a.value else None) if type(a) is c_void_p else a.value if type(a) is c_int else a
@@ -99,7 +102,7 @@ def _p(t):
 class NativeBackend:
     name = "native"
     lays_out_rows = True         # grouped products of many places take scratch for gathered rows (kernels.moe_wants_rows)
-    _recording, _record_lock = None, threading.Lock()
+    _record_lock = threading.Lock()
 
     def __init__(self):
         if not torch.cuda.is_available():
@@ -146,16 +149,18 @@ class NativeBackend:
     def record(self, run, tensors):
         """``run()`` with its launches written down: (what it returned, the recording); the recording is None where one of this
         backend's functions isn't the one written here (what has taken its place would not see the launches made again), and while
-        another recording is made.  The recording stands in the library's place meanwhile, so that a call costs nothing at other times;
-        other threads' calls go through it unrecorded."""
+        another recording is made.  The recording stands in the places of the library and of ``_check`` meanwhile, so that a call costs
+        nothing at other times; other threads' calls go through it unrecorded."""
         if not (_written.holds() and _written.names.isdisjoint(vars(self))) or not self._record_lock.acquire(blocking=False):
             return run(), None
         lib, before = self.lib, self.launches
-        rec = self.lib = self._recording = Recording(self, tensors)
+        rec = self.lib = Recording(self, tensors)
+        self._check = rec.check
         try:
             out = run()
         finally:
-            self.lib, self._recording = lib, None
+            self.lib = lib
+            del self._check
             self._record_lock.release()
         rec.count = self.launches - before
         return out, rec
@@ -169,9 +174,6 @@ class NativeBackend:
     def _check(self, rc: int, what: str):
         if rc != 0:
             raise KernelError(f"{what}: {self.lib.hfb_last_error().decode()} (status {rc})")
-        rec = self._recording
-        if rec is not None and rec.thread == threading.get_ident():
-            rec.add(what)
         self.launches += 1
 
     @staticmethod
