@@ -83,6 +83,11 @@ def backend():
     return _backend
 
 
+def _names(cls):
+    """A class's names but for what Python notes on classes by itself, when one is copied or asked for its annotations."""
+    return frozenset(vars(cls)) - {"__slotnames__", "__annotations__", "__abstractmethods__"}
+
+
 class Written:
     """The functions of some classes and modules as they were when this was made, for code that passes them by: what has been put
     in one's place since (a probe, a wrapper that counts) wants to be called."""
@@ -92,7 +97,7 @@ class Written:
         for s in spaces:
             own = {n: f for n, f in vars(s).items() if callable(f) or isinstance(f, (property, staticmethod, classmethod))}
             # (a class may get a function of a name that only its bases had; a module's new names are nobody's)
-            self._kept.append((s, len(vars(s)) if isinstance(s, type) else None, tuple(own), tuple(own.values()), vars(s)))
+            self._kept.append((s, _names(s) if isinstance(s, type) else None, tuple(own), tuple(own.values()), vars(s)))
         self.names = frozenset(n for k in self._kept for n in k[2])
         self.found = {}                                   # a class's functions by name, its bases' behind its own
         for _, _, names, functions, _ in reversed(self._kept):
@@ -107,8 +112,8 @@ class Written:
         return one
 
     def holds(self) -> bool:
-        return all((size is None or len(space) == size) and tuple(map(space.get, names)) == functions
-                   for _, size, names, functions, space in self._kept)
+        return all((had is None or len(space) == len(had) or _names(s) == had) and tuple(map(space.get, names)) == functions
+                   for s, had, names, functions, space in self._kept)
 
 
 def recorder():

@@ -9,6 +9,7 @@ from __future__ import annotations
 import operator
 import os
 from dataclasses import dataclass
+from functools import lru_cache
 from typing import Dict, List, Optional
 
 import torch
@@ -53,7 +54,15 @@ class Layer:
         return {"post1": self.post1, "post2": self.post2} if self.post1 is not None else {}
 
 
+@lru_cache(maxsize=64)
+def _written(*classes) -> kernels.Written:
+    """The functions of parts' classes as they were written (kept here and not by the models, which can be copied and stored)."""
+    return kernels.Written.together(c.written for c in classes)
+
+
 class Model:
+    _alike = _watched = ()            # what is found when the weights are bound
+
     def __init__(self, config: ModelConfig, run_dtype: torch.dtype = torch.bfloat16,
                  device: torch.device = torch.device("cuda:0"), plan: Optional[ModelPlan] = None):
         if run_dtype not in (torch.bfloat16, torch.float32):
@@ -78,7 +87,6 @@ class Model:
         self.final_norm = make_part("norm", p.final_norm)
         self.head = make_part("head", p.head)
         self.bound = False
-        self._alike, self._watched = [], []
         self.files: List[str] = []            # the weight files this model was loaded from
 
     # ---- weights ------------------------------------------------------------------------
@@ -150,12 +158,12 @@ class Model:
         # layers and parts as they were, and the functions of their classes
         self._watched = list({id(o): o for o in watched}.values())
         self._changes_then, self._layers_then = [o.changes for o in self._watched], list(self.layers)
-        self._written = kernels.Written.together(c.written for c in {type(o): None for o in self._watched if isinstance(o, Part)})
+        self._classes = tuple(dict.fromkeys(type(o) for o in self._watched if isinstance(o, Part)))
 
     def _alike_now(self) -> Optional[List[Optional[int]]]:
         """``_alike``, None where no entries are.  What has been changed since the weights were bound (an attribute of a part, a
         function put over one of its own, another part in its place) is alike with nothing: its own code runs."""
-        if not self._watched or not self._written.holds():
+        if not self._watched or not _written(*self._classes).holds():
             return None
         if [o.changes for o in self._watched] == self._changes_then and len(self.layers) == len(self._layers_then) and \
                 all(map(operator.is_, self.layers, self._layers_then)):

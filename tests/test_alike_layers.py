@@ -249,6 +249,22 @@ def test_a_block_with_state_of_its_own_is_alike_with_none(emu):
     assert torch.equal(_steps(model), want)
 
 
+def test_copies_of_a_model(emu):
+    """A model can be copied and stored; a copy's layers are alike among themselves, and what is changed in it counts there only."""
+    import copy
+    import pickle
+    model = _model()
+    want = _steps(model, record=False)
+    for again in (copy.deepcopy(model), pickle.loads(pickle.dumps(model)), copy.copy(model)):
+        emu.replayed = 0
+        assert torch.equal(_steps(again), want) and emu.replayed == 3 * 3
+        if again.layers is not model.layers:
+            again.layers[2].mixer.scale = 0.9
+            other = _steps(again, record=False)
+            assert not torch.equal(other, want) and torch.equal(_steps(again), other)
+            assert torch.equal(_steps(model), want)
+
+
 def test_only_parts_that_may_be_alike_count_their_changes(emu):
     """Counting costs every attribute of every part that is made; a class that sets attributes its own way is alike with none."""
     from hfcpu_b200.parts.latent_attention import LatentAttention
